@@ -20,6 +20,7 @@
 //     ks_hamiltonian.hpp:166-172);
 //   * EPI_LAPL_ADD: out = fft + lapl(G)*psi_fourier (laplacian_add, laplacian.hpp:24-38).
 
+#include "fft2_lengths.h"
 #include "fft_common.cuh"
 
 namespace inqb {
@@ -148,17 +149,10 @@ void launch_fft_pass(Ctx &ctx, const Basis &b, const PassArgs<R> &a, int prologu
   else throw Error(INQB_ERR_UNSUPPORTED, "unsupported FFT pass fusion");
 }
 
-// N2 of the two-level split when the specialised TMA kernels (fft2.cuh) run every pass along `axis` for
-// S states of elem_bytes each (the conditions of v2::launch), else 0.
+// N2 of the two-level split when the specialised kernels (fft2.cuh) run every pass along `axis` for S states
+// of elem_bytes each in their storage type, else 0.
 int fft2_perm_n2(const Ctx &ctx, const Basis &b, int S, int elem_bytes, int axis) {
-  if (ctx.fft_impl == 1) return 0;
-  const int n = b.n[axis];
-  if (n != 24 && n != 32 && n != 40 && n != 48 && n != 64 && n != 72 && n != 96 && n != 120 && n != 128) return 0;
-  // rows that are not 16-byte multiples: single-precision orbitals only (the producer-warp kernels copy
-  // them); the caller keeps natural order when the arithmetic is not single precision
-  if ((size_t(S) * elem_bytes) % 16 != 0 && elem_bytes != 8) return 0;
-  if (S < 256 / elem_bytes) return 0;
-  return n / 8;
+  return v2::covers(ctx, b, S, elem_bytes, axis) ? v2::split_n2(b.n[axis]) : 0;
 }
 
 template void launch_fft_pass<double>(Ctx &, const Basis &, const PassArgs<double> &, int, int);

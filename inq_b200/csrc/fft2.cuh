@@ -1,7 +1,7 @@
 // Persistent, TMA-pipelined batched FFT pass for compile-time line lengths.
 //
 // Same tile as fft.cu -- one grid line of N points times W consecutive states,
-// 256-byte rows -- but:
+// 256-byte rows (or W consecutive columns of a flattened view; whole z-lines in fftz_kernel) -- but:
 //   * tiles stream through an NS-stage shared-memory ring: one elected thread
 //     issues cp.async.bulk.tensor (TMA) loads NS tiles ahead and a TMA store per
 //     finished tile, so HBM traffic overlaps the arithmetic of the other stages;
@@ -17,6 +17,7 @@
 
 #include <cuda.h>
 
+#include "fft2_lengths.h"
 #include "fft_common.cuh"
 #include "ptx.cuh"
 
@@ -35,15 +36,10 @@ constexpr bool is_perm(int v) { return v >= FWD_PERM; }
 constexpr bool has_aux(int v) { return base_var(v) == INV_FINAL || v == FWD_LAPLADD; }
 
 template <int N> struct Split { static constexpr int N1 = 0, N2 = 0; };
-template <> struct Split<24> { static constexpr int N1 = 8, N2 = 3; };
-template <> struct Split<32> { static constexpr int N1 = 8, N2 = 4; };
-template <> struct Split<40> { static constexpr int N1 = 8, N2 = 5; };
-template <> struct Split<48> { static constexpr int N1 = 8, N2 = 6; };
-template <> struct Split<64> { static constexpr int N1 = 8, N2 = 8; };
-template <> struct Split<72> { static constexpr int N1 = 8, N2 = 9; };
-template <> struct Split<96> { static constexpr int N1 = 8, N2 = 12; };
-template <> struct Split<120> { static constexpr int N1 = 8, N2 = 15; };
-template <> struct Split<128> { static constexpr int N1 = 8, N2 = 16; };
+#define INQB_X(N, A, B) \
+  template <> struct Split<N> { static constexpr int N1 = A, N2 = B; };
+INQB_FFT2_LENGTHS(INQB_X)
+#undef INQB_X
 
 constexpr int first_factor(int M) {
   const int f[6] = {8, 4, 2, 3, 5, 7};
@@ -487,19 +483,26 @@ __device__ __forceinline__ void col_inverse_inplace(T *__restrict__ buf, const T
   }
 }
 
-// The x pass of the real-space operator in place: forward transform, per-frequency factor fac[m],
+// The x pass of the real-space operator in place: forward transform, per-frequency factor f[m],
 // inverse transform.  The inverse runs the forward's two steps transposed (step B first, with
 // conjugate twiddles, then step A), so it starts from the forward's k1-major output and every step
 // writes the rows it read: three shared-memory sweeps and two barriers, no transposition.
 //   forward A: N1-point DFTs down the columns j2, twiddle W_N^{j2 k1}
-//   forward B, factor, inverse B: N2-point DFT along row k1, times fac[k1 + N1 k2], inverse
+//   forward B, factor, inverse B: N2-point DFT along row k1, times f[k1 + N1 k2], inverse
 //     N2-point DFT, twiddle W_N^{-j2 k1} (rows of up to 12 points batched two items at a time)
 //   inverse A: inverse N1-point DFTs down the columns j2, natural order
+// `f` holds the factors of the thread's column: W divides NT, so a thread keeps one column through all steps.
+// Rows batched per thread in the middle step: 24 points at most (two transforms per row; more would spill).
+template <int N, int W, int NT> constexpr int kin_batch() {
+  static_assert(NT % W == 0, "a thread works on one column of the tile");
+  constexpr int n = (W * Split<N>::N1 + NT - 1) / NT, most = 24 / Split<N>::N2;
+  return n < most ? n : (most > 1 ? most : 1);
+}
 template <int N, int W, int NT, typename T, typename Epi>
 __device__ __forceinline__ void tile_kin_inplace(T *__restrict__ buf, const T *__restrict__ tw,
-                                                 const decltype(T::x) *__restrict__ fac, int wsplit, Epi epi) {
+                                                 const decltype(T::x) *__restrict__ f, Epi epi) {
   constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-  constexpr int IB = N2 <= 12 ? (W * N1 + NT - 1) / NT : 1;
+  constexpr int IB = kin_batch<N, W, NT>();
   col_forward_inplace<N, W, NT, T>(buf, tw);
   csync<NT>();
   for (int it0 = threadIdx.x; it0 < W * N1; it0 += IB * NT) {
@@ -518,7 +521,6 @@ __device__ __forceinline__ void tile_kin_inplace(T *__restrict__ buf, const T *_
       const int it = it0 + b * NT;
       if (it < W * N1) {
         const int w = it % W, k1 = it / W;
-        const auto *f = fac + (w >= wsplit ? N : 0);  // the column's line
         dft<N2, +1, N>(r[b], tw);
 #pragma unroll
         for (int k2 = 0; k2 < N2; k2++) r[b][k2] = cscale(r[b][k2], f[k1 + N1 * k2]);
@@ -637,22 +639,21 @@ __device__ __forceinline__ void col_inverse(const TC *work, const TC *__restrict
   }
 }
 
-// Forward transform, per-frequency factor fac[m], inverse transform of one [N][W] tile (the x pass of
+// Forward transform, per-frequency factor f[m], inverse transform of one [N][W] tile (the x pass of
 // the real-space operator), with the arithmetic in a separate buffer `work` (wider type than the
 // tile); the in-place form for equal types is tile_kin_inplace.  The inverse runs the forward's two steps transposed (step B first, with
 // conjugate twiddles, then step A), so it starts from the forward's k1-major output and every step
 // writes the addresses it read: three shared-memory sweeps and two barriers, no transposition.
 //   forward A: N1-point DFTs down the columns j2, twiddle W_N^{j2 k1}           (asrc -> work)
-//   forward B, factor, inverse B: N2-point DFT along row k1, times fac[k1 + N1 k2], inverse
+//   forward B, factor, inverse B: N2-point DFT along row k1, times f[k1 + N1 k2], inverse
 //     N2-point DFT, twiddle W_N^{-j2 k1}                                      (work, in place)
 //   inverse A: inverse N1-point DFTs down the columns j2; x[j2 + N2 j1] goes to put(m, w, value)
 // `asrc` may be `work` itself.  No barrier follows the last step.
 template <int N, int W, int NT, typename TC, typename SA, typename Put>
 __device__ __forceinline__ void tile_dft_kin(const SA *asrc, TC *work, const TC *__restrict__ tw,
-                                             const decltype(TC::x) *fac, int wsplit, Put put) {
+                                             const decltype(TC::x) *f, Put put) {
   constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-  // rows of up to 12 points are batched (two transforms per row keep longer rows one at a time)
-  constexpr int IB = N2 <= 12 ? (W * N1 + NT - 1) / NT : 1;
+  constexpr int IB = kin_batch<N, W, NT>();
   col_forward<N, W, NT, TC>(asrc, work, tw);
   csync<NT>();
   for (int it0 = threadIdx.x; it0 < W * N1; it0 += IB * NT) {
@@ -671,7 +672,6 @@ __device__ __forceinline__ void tile_dft_kin(const SA *asrc, TC *work, const TC 
       const int it = it0 + b * NT;
       if (it < W * N1) {
         const int w = it % W, k1 = it / W;
-        const auto *f = fac + (w >= wsplit ? N : 0);  // the column's line
         dft<N2, +1, N>(r[b], tw);
 #pragma unroll
         for (int k2 = 0; k2 < N2; k2++) r[b][k2] = cscale(r[b][k2], f[k1 + N1 * k2]);
@@ -701,6 +701,7 @@ struct Geom2 {
                     // cp.async loads and plain stores instead of TMA (two stages, second tiles per stage)
   int flat;         // y and x passes over flattened columns (below); nsb is then the column blocks per row
   long long ncols;  // flat: columns per row, nz*S (y pass) or ny*nz*S (x pass)
+  int flines;       // lines whose factors a tile may need (an even number: what follows stays 8-byte aligned)
 };
 
 // Flattened columns.  A y (x) transform acts on every column of the [nx][ny][nz*S] ([nx][ny*nz*S]) view
@@ -709,8 +710,8 @@ struct Geom2 {
 // (odd counts too, whose point rows are not 16-byte multiples, and counts that leave the last state block
 // of a line part-empty), and only the last tile of each row runs past its end (TMA fills the loads with
 // zeros and clips the stores).  With S a multiple of W the tiles, and their order, are those of the
-// (line, state block) decomposition.  The kinetic factor of a column depends on its (y, z) line; with
-// S >= W a tile's columns lie on at most two lines.
+// (line, state block) decomposition.  The kinetic factor of a column depends on its (y, z) line; a tile's
+// columns lie on at most (W - 1) / S + 2 lines, two when S >= W.
 
 template <int VAR> constexpr int dir_first() { return (base_var(VAR) == INV_STORE || base_var(VAR) == INV_FINAL) ? -1 : +1; }
 
@@ -790,8 +791,8 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
   TC *exch = reinterpret_cast<TC *>(aux_ring + size_t(aux1 ? 1 : NS) * naux * TILE);  // one tile when SPLIT
   constexpr int TWN = tw_entries<CR>(N);
   TC *tw = exch + (SPLIT ? TILE : 0);                                // twiddles (high, then low parts)
-  CR *linev = reinterpret_cast<CR *>(tw + TWN);                      // N per-point factors of the current line
-  uint64_t *bar = reinterpret_cast<uint64_t *>(tw + TWN + N);        // NS "tile loaded" barriers (8-byte aligned)
+  CR *linev = reinterpret_cast<CR *>(tw + TWN);                      // N per-point factors per line of the tile
+  uint64_t *bar = reinterpret_cast<uint64_t *>(linev + gg.flines * N);  // NS "tile loaded" barriers (8-byte aligned)
   uint64_t *done = bar + NS;                                         // NS "tile computed" barriers (producer warp)
   uint64_t *abar = done + NS;                                        // "second input tiles loaded"
   volatile int *abort_flag = reinterpret_cast<volatile int *>(abar + 1);
@@ -971,14 +972,15 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
     const long long pbase = la * g.sa + lb * g.sb;
 
     // per-point factors of this line (consumed after the first barrier of the transform); flattened
-    // columns: of the tile's first line at linev[0, N) and, from column wsplit on, of the next at [N, 2N)
-    int wsplit = W;
+    // columns: of every line the tile's columns lie on, one after the other; lv: those of the thread's column
+    const CR *lv = linev;
     if constexpr (VAR == MID_KIN || VAR == FWD_LAPLADD) {
       if (gg.flat) {
         // 32-bit divisions: a view row has fewer than 2^31 words (the host checks it)
-        const int col0 = int(t % gg.nsb) * W, l0 = col0 / a.S, nlines = g.n[1] * g.n[2];
-        wsplit = (l0 + 1) * a.S - col0 < W ? (l0 + 1) * a.S - col0 : W;
-        const int nl = (wsplit < W && l0 + 1 < nlines) ? 2 : 1;
+        const int col0 = int(t % gg.nsb) * W, l0 = col0 / a.S;
+        const int last = col0 + W - 1 < int(gg.ncols) ? col0 + W - 1 : int(gg.ncols) - 1;
+        const int nl = last / a.S - l0 + 1, mine = col0 + int(threadIdx.x % W);
+        lv = linev + N * ((mine < last ? mine : last) / a.S - l0);
         for (int e = threadIdx.x; e < nl * N; e += NT) {
           const int l = l0 + e / N;  // x-line (y, z) = (l / nz, l % nz)
           const int ly = l / g.n[2];
@@ -1027,7 +1029,7 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
         }
       }
       if (scaled) v = kscale(v, a.scale);
-      if constexpr (base_var(VAR) == INV_FINAL || VAR == FWD_LAPLADD) v = cadd(v, cscale(conv<TC>(aux[m * W + w]), linev[m]));
+      if constexpr (base_var(VAR) == INV_FINAL || VAR == FWD_LAPLADD) v = cadd(v, cscale(conv<TC>(aux[m * W + w]), lv[m]));
       if constexpr (AUX) {
         if (horner) return cadd(base[m * W + w], cmul(a.hc, conv<T>(v)));
       }
@@ -1042,7 +1044,7 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
       static_assert(!is_perm(VAR), "digit-reversed passes run with equal storage and arithmetic types");
       if constexpr (VAR == MID_KIN) {
         // forward, multiply by the kinetic factor, backward
-        tile_dft_kin<N, W, NT, TC>(buf, exch, tw, linev, wsplit, put_out);
+        tile_dft_kin<N, W, NT, TC>(buf, exch, tw, lv, put_out);
       } else {
         tile_dft<N, D, W, NT, false, TC>(buf, exch, tw, pre, put_out);
       }
@@ -1056,8 +1058,8 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
       // plain passes (no scaling, no accumulators) store the transform's values as they are
       const bool plain = !AUX && !scaled;
       if constexpr (VAR == MID_KIN) {
-        if (plain) tile_kin_inplace<N, W, NT, T>(buf, twt, linev, wsplit, Identity());
-        else tile_kin_inplace<N, W, NT, T>(buf, twt, linev, wsplit, epi_out);
+        if (plain) tile_kin_inplace<N, W, NT, T>(buf, twt, lv, Identity());
+        else tile_kin_inplace<N, W, NT, T>(buf, twt, lv, epi_out);
       } else if constexpr (VAR == INV_FINAL_PERM) {
         tile_inv_perm_inplace<N, W, NT, T>(buf, twt, epi_out);
       } else if constexpr (VAR == FWD_PERM || VAR == INV_PERM) {
@@ -1070,6 +1072,8 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
       } else if constexpr (AUX) {
         // the epilogue (V psi or the Laplacian term, Taylor accumulators) in the transform's last step
         tile_dft_inplace<N, D, W, NT, T>(buf, twt, epi_out);
+      } else if (VAR == INV_STORE && scaled) {
+        tile_dft_inplace<N, D, W, NT, T>(buf, twt, [&](int, int, T v) { return kscale(v, a.scale); });
       } else {
         tile_dft_inplace<N, D, W, NT, T>(buf, twt, Identity());
         if (!plain) {
@@ -1114,6 +1118,243 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
   if (!WS && threadIdx.x == 0) {
     drain();
     bulk_wait0();
+  }
+}
+
+
+// ------------------------------------------------------------------ z passes over whole lines
+
+// A z-line's points follow one another in memory, so `lpt` whole lines with all their states are one
+// contiguous chunk, whatever the state count: one bulk copy loads it, odd counts (whose point rows no
+// tensor map describes) and few states included, and no tile slot is empty.  The tiles of fft2_kernel
+// leave up to a whole state block of each line empty, and move odd single-precision counts with 8-byte
+// copies of the compute threads.
+//
+// In the chunk [line][point][state] the first step's items (j2, s) and the second step's (k1, s) of a line
+// are consecutive too: item i of a column step touches i + j1 N2 S, so consecutive threads read consecutive
+// elements and only the twiddles need the item's (j2, s), one multiplication by a reciprocal.  The first
+// step works in shared memory in place, the second goes straight to global memory with its epilogue (a
+// warp stores consecutive elements); the second inputs of an epilogue are read there the same way, before
+// the step's shared-memory loads, so they need no tile of their own.
+//
+// Bound by HBM: one transit in and one out (and the second inputs).  Two stages per CTA and 10 to 18 warps
+// per SM cover the latency; see zlines_of for the chunk and thread counts.  Measured: 72^3 x 99 single,
+// forward 206 -> 95 us (6.2 TB/s) and final 354 -> 183 us against the 8-byte copies; 40^3 x 33 double, forward
+// 22.8 -> 12.4 and final Horner pass 46.7 -> 31.0 us against 16-state tiles (48 slots for 33 states).  Rows
+// that are whole 256-byte tiles keep the TMA tiles of fft2_kernel, which leave nothing empty either.
+struct GeomZ {
+  long long lines;           // nx * ny
+  int lpt, stages;
+  int ntiles;
+  uint32_t mag_s, mag_a, mag_b;  // reciprocals of S, N2 S (items per line of a column step), N1 S
+};
+// floor(i / d) for i d < 2^32 with m = ceil(2^32 / d); m = 0 stands for d = 1
+__device__ __forceinline__ int div_by(int i, uint32_t m) { return m ? int(__umulhi(uint32_t(i), m)) : i; }
+
+template <typename R> constexpr int zl_max_threads() { return (sizeof(R) == 8 ? 320 : 480) + 32; }
+
+template <typename R, int N, int VAR>
+__global__ void __launch_bounds__(zl_max_threads<R>()) fftz_kernel(PassArgs<R> a, GeomZ gz,
+                                                                  const C2<R> *__restrict__ twg, int *err) {
+  using T = C2<R>;
+  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
+  constexpr int TWN = tw_entries<R>(N);
+  constexpr int D = dir_first<VAR>();
+  constexpr bool FINAL = base_var(VAR) == INV_FINAL;
+  constexpr bool LINEV = FINAL || VAR == FWD_VPSI;
+  const int NT = int(blockDim.x) - 32;  // compute threads; the last warp's lane 0 issues the loads
+  const int S = a.S, NS = gz.stages;
+  const int line = N * S;               // elements per line
+  const int chunk = gz.lpt * line;
+
+  extern __shared__ __align__(1024) unsigned char smem[];
+  T *ring = reinterpret_cast<T *>(smem);
+  T *tw = ring + size_t(NS) * chunk;
+  R *linev = reinterpret_cast<R *>(tw + TWN);  // V + shift of the chunk's points
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + ((size_t(NS) * chunk * sizeof(T) + TWN * sizeof(T) +
+                                                         size_t(gz.lpt) * N * sizeof(R) + 15) & ~size_t(15)));
+  uint64_t *done = full + NS;
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(done + NS);
+
+  for (int i = threadIdx.x; i < TWN; i += blockDim.x) tw[i] = twg[i];
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < NS; s++) {
+      mbar_init(&full[s], 1);
+      mbar_init(&done[s], NT);
+    }
+    mbar_init_fence();
+  }
+  __syncthreads();
+
+  auto wait_bar = [&](uint64_t *b, uint32_t parity) -> bool {
+    const uint64_t t0 = global_ns();
+    while (!mbar_try_wait(b, parity)) {
+      if (*abort_flag) return false;
+      if (global_ns() - t0 > 2000000000ull) {
+        *abort_flag = 1;
+        atomicExch(err, 1);
+        return false;
+      }
+    }
+    return true;
+  };
+  auto lines_of = [&](int t) {
+    const long long left = gz.lines - (long long)t * gz.lpt;
+    return left < gz.lpt ? int(left) : gz.lpt;
+  };
+
+  if (int(threadIdx.x) >= NT) {
+    if (int(threadIdx.x) == NT) {
+      int k = 0;
+      for (int t = blockIdx.x; t < gz.ntiles; t += gridDim.x, k++) {
+        const int st = k % NS;
+        if (k >= NS && !wait_bar(&done[st], uint32_t(k / NS - 1) & 1u)) break;
+        const uint32_t bytes = uint32_t(lines_of(t)) * uint32_t(line) * uint32_t(sizeof(T));
+        mbar_expect_tx(&full[st], bytes);
+        ptx::bulk_load(ring + size_t(st) * chunk, a.in + (long long)t * chunk, bytes, &full[st]);
+      }
+      // after an aborted wait the compute threads may leave early: no load may still land in the CTA's
+      // shared memory then (on the normal path these phases are complete)
+      for (int i = k - NS < 0 ? 0 : k - NS; i < k; i++)
+        ptx::mbar_wait_bounded(&full[i % NS], uint32_t(i / NS) & 1u, 2000000000ull);
+    }
+    return;
+  }
+
+  auto sync = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(NT) : "memory"); };
+  auto sync_or = [&](int v) -> bool {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r)
+                 : "r"(v), "r"(NT)
+                 : "memory");
+    return r != 0;
+  };
+  const bool horner = FINAL && a.hbase != nullptr;
+  const bool scaled = a.scale != 1.0;
+  const int tid = threadIdx.x, colS = N2 * S, rowS = N1 * S;
+  int i = 0;
+  for (int t = blockIdx.x; t < gz.ntiles; t += gridDim.x, i++) {
+    const int st = i % NS;
+    const bool ok = wait_bar(&full[st], uint32_t(i / NS) & 1u);
+    if (sync_or(!ok || *abort_flag)) break;
+    T *__restrict__ buf = ring + size_t(st) * chunk;
+    const int nl = lines_of(t);
+    const long long g0 = (long long)t * chunk;  // the chunk's first element
+    T *__restrict__ out = a.out + g0;
+    if constexpr (LINEV) {
+      const long long p0 = (long long)t * gz.lpt * N;
+      const bool masked = VAR == FWD_VPSI && a.nl_offs != nullptr;
+      for (int m = tid; m < nl * N; m += NT) {
+        const long long pt = p0 + m;
+        // points with sphere hits already hold (V + shift) psi + nonlocal
+        linev[m] = masked && a.nl_offs[pt + 1] > a.nl_offs[pt] ? R(1) : a.V[pt * a.nspin + a.spin] + a.vshift;
+      }
+      if constexpr (VAR == FWD_VPSI) sync();
+    }
+
+    if constexpr (VAR == INV_PERM || VAR == INV_FINAL_PERM) {
+      // rows first (digit-reversed input), then columns in natural order
+      for (int it = tid; it < nl * rowS; it += NT) {
+        const int l = nl > 1 ? div_by(it, gz.mag_b) : 0, r = it - l * rowS;
+        const int k1 = div_by(r, gz.mag_s);
+        T *p = buf + l * line + k1 * colS + (r - k1 * S);
+        T v[N2];
+#pragma unroll
+        for (int k2 = 0; k2 < N2; k2++) v[k2] = p[k2 * S];
+        dft<N2, -1, N>(v, tw);
+        if (k1 > 0) {
+#pragma unroll
+          for (int j2 = 1; j2 < N2; j2++) v[j2] = twmul<-1, N>(v[j2], tw, j2 * k1);
+        }
+#pragma unroll
+        for (int j2 = 0; j2 < N2; j2++) p[j2 * S] = v[j2];
+      }
+      sync();
+      for (int it = tid; it < nl * colS; it += NT) {
+        const int l = nl > 1 ? div_by(it, gz.mag_a) : 0, r = it - l * colS;
+        const int e0 = l * line + r;
+        T x[FINAL ? N1 : 1], h[FINAL ? N1 : 1];
+        if constexpr (FINAL) {
+#pragma unroll
+          for (int j1 = 0; j1 < N1; j1++) x[j1] = a.psi[g0 + e0 + j1 * colS];
+          if (horner) {
+#pragma unroll
+            for (int j1 = 0; j1 < N1; j1++) h[j1] = a.hbase[g0 + e0 + j1 * colS];
+          }
+        }
+        T v[N1];
+#pragma unroll
+        for (int k1 = 0; k1 < N1; k1++) v[k1] = buf[e0 + k1 * colS];
+        dft<N1, -1, N>(v, tw);
+        if constexpr (FINAL) {
+          const R *lv = linev + l * N + div_by(r, gz.mag_s);
+#pragma unroll
+          for (int j1 = 0; j1 < N1; j1++) {
+            T o = scaled ? kscale(v[j1], a.scale) : v[j1];
+            o = cadd(o, cscale(x[j1], lv[j1 * N2]));
+            if (horner) o = cadd(h[j1], cmul(a.hc, o));
+            out[e0 + j1 * colS] = o;
+          }
+        } else {
+#pragma unroll
+          for (int j1 = 0; j1 < N1; j1++) out[e0 + j1 * colS] = scaled ? kscale(v[j1], a.scale) : v[j1];
+        }
+      }
+    } else {
+      // columns first, then rows: natural order, or rows of digit-reversed frequencies
+      for (int it = tid; it < nl * colS; it += NT) {
+        const int l = nl > 1 ? div_by(it, gz.mag_a) : 0, r = it - l * colS;
+        const int j2 = div_by(r, gz.mag_s);
+        T *p = buf + l * line + r;
+        T v[N1];
+#pragma unroll
+        for (int j1 = 0; j1 < N1; j1++) v[j1] = p[j1 * colS];
+        if constexpr (VAR == FWD_VPSI) {
+          const R *lv = linev + l * N + j2;
+#pragma unroll
+          for (int j1 = 0; j1 < N1; j1++) v[j1] = cscale(v[j1], lv[j1 * N2]);
+        }
+        dft<N1, D, N>(v, tw);
+#pragma unroll
+        for (int k1 = 1; k1 < N1; k1++) v[k1] = twmul<D, N>(v[k1], tw, j2 * k1);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; k1++) p[k1 * colS] = v[k1];
+      }
+      sync();
+      for (int it = tid; it < nl * rowS; it += NT) {
+        const int l = nl > 1 ? div_by(it, gz.mag_b) : 0, r = it - l * rowS;
+        const int k1 = div_by(r, gz.mag_s), s = r - k1 * S;
+        const int e0 = l * line + s;
+        const T *p = buf + e0 + k1 * colS;
+        T x[FINAL ? N2 : 1], h[FINAL ? N2 : 1];
+        if constexpr (FINAL) {
+#pragma unroll
+          for (int k2 = 0; k2 < N2; k2++) x[k2] = a.psi[g0 + e0 + (k1 + N1 * k2) * S];
+          if (horner) {
+#pragma unroll
+            for (int k2 = 0; k2 < N2; k2++) h[k2] = a.hbase[g0 + e0 + (k1 + N1 * k2) * S];
+          }
+        }
+        T v[N2];
+#pragma unroll
+        for (int j2 = 0; j2 < N2; j2++) v[j2] = p[j2 * S];
+        dft<N2, D, N, (sizeof(R) == 4 && D > 0)>(v, tw);
+#pragma unroll
+        for (int k2 = 0; k2 < N2; k2++) {
+          const int m = VAR == FWD_PERM ? k2 + N2 * k1 : k1 + N1 * k2;
+          T o = scaled ? kscale(v[k2], a.scale) : v[k2];
+          if constexpr (FINAL) {
+            o = cadd(o, cscale(x[k2], linev[l * N + m]));
+            if (horner) o = cadd(h[k2], cmul(a.hc, o));
+          }
+          out[e0 + m * S] = o;
+        }
+      }
+    }
+    fence_proxy_async();
+    mbar_arrive(&done[st]);  // every read of the stage is done: it may be refilled
   }
 }
 
@@ -1184,7 +1425,10 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
   const int naux = has_aux(VAR) ? (a.hbase ? 2 : 1) : 0;
   constexpr bool SPLIT = sizeof(CR) > sizeof(R);
   constexpr int NT = block_threads_of<R, CR, N, VAR, WIDE>();
-  const size_t fixed = (SPLIT ? size_t(N) * W * sizeof(TC) : 0) + size_t(tw_entries<CR>(N) + N) * sizeof(TC) + 64 + 16 * 8;
+  // lines whose factors a flattened tile needs: at most (W - 1) / S + 2 consecutive ones
+  gg.flines = ((VAR == MID_KIN || VAR == FWD_LAPLADD) && gg.flat && a.S < W) ? ((W - 1) / a.S + 3) / 2 * 2 : 2;
+  const size_t fixed = (SPLIT ? size_t(N) * W * sizeof(TC) : 0) + size_t(tw_entries<CR>(N)) * sizeof(TC) +
+                       size_t(gg.flines) * N * sizeof(CR) + 64 + 16 * 8;
   // shared memory per CTA: ~113 KB (two CTAs per SM) for the FP64 streaming passes; ~56 KB (four per SM)
   // for the wide-arithmetic, the kinetic and the producer-warp (single-precision) passes, whose
   // arithmetic needs more warps to hide latency (96^3 x 256 single: 3.81 ms per H against 3.89 with
@@ -1205,7 +1449,6 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
   if (gg.cpa) ns = 2;
   gg.stages = ns;
   if (gg.flat) {
-    INQB_REQUIRE(VAR != MID_KIN || a.S >= W, INQB_ERR_UNSUPPORTED, "flattened kinetic tiles span more than two lines");
     gg.nsb = (gg.ncols + W - 1) / W;
     gg.ntiles = gg.axis == 1 ? (long long)b.n[0] * gg.nsb : gg.nsb;
   } else {
@@ -1241,7 +1484,8 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
   if (gg.flat) {
     mi = flat_map(a.in, b, gg.ncols, cwords, gg.axis, W);
     mo = flat_map(a.out, b, gg.ncols, cwords, gg.axis, W);
-    mx = mb = mi;
+    mx = has_aux(VAR) ? flat_map(a.psi, b, gg.ncols, cwords, gg.axis, W) : mi;
+    mb = mi;
   } else if (!gg.cpa) {
     mi = orbital_map(a.in, b, a.S, cwords, gg.axis, W);
     mo = orbital_map(a.out, b, a.S, cwords, gg.axis, W);
@@ -1308,8 +1552,50 @@ template <typename R> bool single_arith(const Ctx &ctx, const PassArgs<R> &a, in
   return mode == 0 || (mode >= 2 && bv == INV_FINAL) || (mode == 3 && a.axis == 2 && (bv == FWD_STORE || var == FWD_VPSI));
 }
 
+// the z pass over whole lines (fftz_kernel)
+template <typename R, int N, int VAR>
+void launch_zlines(Ctx &ctx, const Basis &b, const PassArgs<R> &a, const ZLines &z) {
+  using T = C2<R>;
+  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
+  GeomZ gz;
+  gz.lines = (long long)b.n[0] * b.n[1];
+  gz.lpt = z.lpt;
+  gz.stages = z.stages;
+  const long long tiles = (gz.lines + z.lpt - 1) / z.lpt;
+  INQB_REQUIRE(tiles < (1LL << 31), INQB_ERR_UNSUPPORTED, "FFT pass has more than 2^31 tiles");
+  gz.ntiles = int(tiles);
+  auto mag = [](uint64_t d) { return d == 1 ? 0u : uint32_t(((1ull << 32) + d - 1) / d); };
+  gz.mag_s = mag(uint64_t(a.S));
+  gz.mag_a = mag(uint64_t(N2) * a.S);
+  gz.mag_b = mag(uint64_t(N1) * a.S);
+  const size_t smem = zlines_smem(N, a.S, int(sizeof(T)), z.lpt, z.stages);
+  auto kern = fftz_kernel<R, N, VAR>;
+  ensure_smem_attr(reinterpret_cast<const void *>(kern), smem);
+  const int ctas = int((ctx.max_smem_optin + 1024) / (smem + 1024));
+  long long grid = (long long)(ctas < 1 ? 1 : (ctas > 8 ? 8 : ctas)) * ctx.num_sms;
+  if (grid > tiles) grid = tiles;
+  const T *tw = reinterpret_cast<const T *>(sizeof(R) == 8 ? b.tw64[2] : b.tw32[2]);
+  kern<<<unsigned(grid), z.threads + 32, smem, ctx.stream>>>(a, gz, tw, ctx.d_err);
+  INQB_CUDA(cudaGetLastError());
+  ctx.launches++;
+}
+
 template <typename R, int N>
 void launch_n(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg, int var) {
+  if (gg.axis == 2 && var != FWD_VPSI && (sizeof(R) == 8 || single_arith(ctx, a, var))) {
+    const ZLines z = zlines_of(ctx, b, a.S, int(sizeof(C2<R>)));
+    if (z.lpt > 0) {
+      switch (var) {
+        case FWD_STORE: launch_zlines<R, N, FWD_STORE>(ctx, b, a, z); return;
+        case INV_STORE: launch_zlines<R, N, INV_STORE>(ctx, b, a, z); return;
+        case INV_FINAL: launch_zlines<R, N, INV_FINAL>(ctx, b, a, z); return;
+        case FWD_PERM: launch_zlines<R, N, FWD_PERM>(ctx, b, a, z); return;
+        case INV_PERM: launch_zlines<R, N, INV_PERM>(ctx, b, a, z); return;
+        case INV_FINAL_PERM: launch_zlines<R, N, INV_FINAL_PERM>(ctx, b, a, z); return;
+        default: break;
+      }
+    }
+  }
   if constexpr (sizeof(R) == 4) {
     const bool single = single_arith(ctx, a, var);
     if (single) {
@@ -1320,17 +1606,26 @@ void launch_n(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg, int var)
       launch_nc<R, float, N>(ctx, b, a, gg, var, wide);
       return;
     }
+    if constexpr (has_wide_arith(N)) launch_nc<R, double, N>(ctx, b, a, gg, var);
+    else throw Error(INQB_ERR_UNSUPPORTED, "no double-precision arithmetic for this line length");
+  } else {
+    launch_nc<R, double, N>(ctx, b, a, gg, var);
   }
-  launch_nc<R, double, N>(ctx, b, a, gg, var);
 }
+
+// one length's kernels, each instantiated in one of the fft2_inst_*.cu files
+#define INQB_X(N, A, B)                                                                                    \
+  extern template void launch_n<float, N>(Ctx &, const Basis &, const PassArgs<float> &, Geom2, int);      \
+  extern template void launch_n<double, N>(Ctx &, const Basis &, const PassArgs<double> &, Geom2, int);
+INQB_FFT2_LENGTHS(INQB_X)
+#undef INQB_X
 
 // Returns false (and does nothing) when the pass is not covered by a specialised kernel.
 template <typename R> bool launch(Ctx &ctx, const Basis &b, const PassArgs<R> &a, int prologue, int epilogue) {
   using T = C2<R>;
   if (ctx.fft_impl == 1) return false;
   const int n = b.n[a.axis];
-  if (n != 24 && n != 32 && n != 40 && n != 48 && n != 64 && n != 72 && n != 96 && n != 120 && n != 128) return false;
-  if (a.S < 256 / int(sizeof(T))) return false;  // fewer states than one 256-byte row: generic kernel
+  if (split_n2(n) == 0) return false;
   int var;
   if (a.mid_kinetic) var = MID_KIN;
   else if (prologue == PRO_VPSI) var = FWD_VPSI;
@@ -1338,19 +1633,18 @@ template <typename R> bool launch(Ctx &ctx, const Basis &b, const PassArgs<R> &a
   else if (epilogue == EPI_LAPL_ADD) var = FWD_LAPLADD;
   else var = a.dir > 0 ? FWD_STORE : INV_STORE;
   if ((var == INV_FINAL && a.dir > 0) || ((var == FWD_VPSI || var == FWD_LAPLADD) && a.dir < 0)) return false;
-  // y and x passes without per-line data over flattened columns (context option fft_flat), when the
-  // rows of the flattened view are 16-byte multiples
-  // (and the 32-bit words of a view row stay below 2^31, the range of a TMA coordinate).  When every tile
-  // width divides the state count (a multiple of 512-byte rows) the two decompositions give the same
-  // tiles, and the line tiles' per-tile index arithmetic is the cheaper (96^3 x 256 single: x pass 0.65
-  // against 0.69 ms), so they are kept there.
-  const long long view_words = (a.axis == 1 ? (long long)b.n[2] : (long long)b.n[1] * b.n[2]) * a.S * (sizeof(T) / 4);
-  const bool flat = ctx.fft_flat && a.axis != 2 && (var == FWD_STORE || var == INV_STORE || var == MID_KIN) &&
-                    (size_t(b.n[2]) * a.S * sizeof(T)) % 16 == 0 && view_words < (1LL << 31) &&
-                    (size_t(a.S) * sizeof(T)) % 512 != 0;
-  // rows that are not 16-byte multiples (an odd number of single-precision states): only the kernels with
-  // a producer warp (single-precision arithmetic) move them, with 8-byte copies; otherwise the generic kernel
-  if (!flat && (size_t(a.S) * sizeof(T)) % 16 != 0 && !(sizeof(R) == 4 && single_arith(ctx, a, var))) return false;
+  const bool same_type = sizeof(R) == 8 || single_arith(ctx, a, var);
+  if (!same_type && !has_wide_arith(n)) return false;
+  // y and x passes over flattened columns (their second input, the Laplacian term's, lies alike)
+  const bool flat = flat_ok(ctx, b, a.S, int(sizeof(T)), a.axis) &&
+                    (var == FWD_STORE || var == INV_STORE || var == MID_KIN || var == FWD_LAPLADD);
+  const bool zl = a.axis == 2 && same_type && var != FWD_VPSI && zlines_of(ctx, b, a.S, int(sizeof(T))).lpt > 0;
+  if (!flat && !zl) {
+    if (a.S < 256 / int(sizeof(T))) return false;  // fewer states than one 256-byte row: generic kernel
+    // rows that are not 16-byte multiples (an odd number of single-precision states): only the kernels with
+    // a producer warp (single-precision arithmetic) move them, with 8-byte copies; otherwise the generic kernel
+    if ((size_t(a.S) * sizeof(T)) % 16 != 0 && !(sizeof(R) == 4 && same_type)) return false;
+  }
   if (a.perm) {
     INQB_REQUIRE(var == FWD_STORE || var == INV_STORE || var == INV_FINAL, INQB_ERR_UNSUPPORTED,
                  "digit-reversed frequency order is only kept by the plain forward and inverse passes");
@@ -1374,15 +1668,9 @@ template <typename R> bool launch(Ctx &ctx, const Basis &b, const PassArgs<R> &a
   gg.cwords = int(sizeof(T) / 4);
   gg.stages = 2;
   switch (n) {
-    case 24: launch_n<R, 24>(ctx, b, a, gg, var); break;
-    case 32: launch_n<R, 32>(ctx, b, a, gg, var); break;
-    case 40: launch_n<R, 40>(ctx, b, a, gg, var); break;
-    case 48: launch_n<R, 48>(ctx, b, a, gg, var); break;
-    case 64: launch_n<R, 64>(ctx, b, a, gg, var); break;
-    case 72: launch_n<R, 72>(ctx, b, a, gg, var); break;
-    case 96: launch_n<R, 96>(ctx, b, a, gg, var); break;
-    case 120: launch_n<R, 120>(ctx, b, a, gg, var); break;
-    default: launch_n<R, 128>(ctx, b, a, gg, var); break;
+#define INQB_X(N, A, B) case N: launch_n<R, N>(ctx, b, a, gg, var); break;
+    INQB_FFT2_LENGTHS(INQB_X)
+#undef INQB_X
   }
   return true;
 }

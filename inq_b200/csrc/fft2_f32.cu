@@ -1,4 +1,4 @@
-// Specialised TMA-pipelined FFT passes, single precision (mixed form).
+// Dispatch of the specialised FFT passes, single precision (mixed form).
 #include "fft2.cuh"
 
 namespace inqb {

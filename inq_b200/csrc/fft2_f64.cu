@@ -1,4 +1,4 @@
-// Specialised TMA-pipelined FFT passes, double precision (plain form).
+// Dispatch of the specialised FFT passes, double precision.
 #include "fft2.cuh"
 
 namespace inqb {
