@@ -12,11 +12,10 @@
 // ks_hamiltonian.hpp:137-180):
 //   * mid_kinetic: forward transform, multiply by factor*(-|G|^2 + gc.G)
 //     (laplacian.hpp:31-36), backward transform -- all in one tile visit;
-//   * EPI_FINAL_REAL: out = scale*fft + (V + shift)*psi + nonlocal(psi) with the
-//     nonlocal term taken from the per-grid-point hit lists (owner computes, no
-//     atomics; projector_all.hpp:276-288) and the 1/N of to_real (transform.hpp:175-181);
+//   * EPI_FINAL_REAL: out = scale*fft + (V + shift)*psi with the 1/N of to_real (transform.hpp:175-181);
 //     optionally a Horner step of a Taylor exponential, out = base + c*out (exponential.hpp:21-34);
-//   * PRO_VPSI: the tile is loaded as (V + shift)*psi + nonlocal (Fourier-form operator,
+//   * PRO_VPSI: the tile is loaded as (V + shift)*psi, but as it is at the points with sphere hits, where
+//     the nonlocal apply has formed (V + shift)*psi + nonlocal (Fourier-form operator,
 //     ks_hamiltonian.hpp:166-172);
 //   * EPI_LAPL_ADD: out = fft + lapl(G)*psi_fourier (laplacian_add, laplacian.hpp:24-38).
 
@@ -54,9 +53,8 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(PassArgs<R> a, Geom g, Ra
       const long long e = pt * a.S + s;
       v = a.in[e];
       if (PRO == PRO_VPSI) {
-        R vv = a.V[pt * a.nspin + a.spin] + a.vshift;
-        v = cscale(v, vv);
-        if (a.nl_offs) v = cadd(v, nl_term<R>(a, pt, s));
+        // points with sphere hits already hold (V + shift) psi + nonlocal
+        if (!(a.nl_offs && a.nl_offs[pt + 1] > a.nl_offs[pt])) v = cscale(v, a.V[pt * a.nspin + a.spin] + a.vshift);
       }
     }
     bufA[p * W + w] = v;
@@ -87,7 +85,6 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(PassArgs<R> a, Geom g, Ra
     if (EPI == EPI_FINAL_REAL) {
       R vv = a.V[pt * a.nspin + a.spin] + a.vshift;
       v = cadd(v, cscale(a.psi[e], vv));
-      if (a.nl_offs) v = cadd(v, nl_term<R>(a, pt, s));
     } else if (EPI == EPI_LAPL_ADD) {
       int ix, iy, iz;
       line_coords(a.axis, la, lb, p, ix, iy, iz);

@@ -411,15 +411,25 @@ struct Identity {
 
 // Natural order in and out: step A (N1-point DFTs down the columns j2, twiddle W_N^{j2 k1}), step B
 // (N2-point DFTs along the rows k1, outputs m = k1 + N1 k2).  Step B reads all its inputs before a
-// barrier and stores after it (it writes other rows than it reads).
+// barrier and stores after it (it writes other rows than it reads).  `pre`: per-point factors applied on load;
+// `scale` likewise (in the first step: a second form of the last one doubles the registers of long FP64 lines).
 template <int N, int DIR, int W, int NT, typename T, typename Epi>
-__device__ __forceinline__ void tile_dft_inplace(T *__restrict__ buf, const T *__restrict__ tw, Epi epi) {
+__device__ __forceinline__ void tile_dft_inplace(T *__restrict__ buf, const T *__restrict__ tw, Epi epi,
+                                                 const decltype(T::x) *pre = nullptr, bool scaled = false,
+                                                 double scale = 1.0) {
   constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
   for (int it = threadIdx.x; it < W * N2; it += NT) {
     const int w = it % W, j2 = it / W;
     T s[N1];
 #pragma unroll
-    for (int j1 = 0; j1 < N1; j1++) s[j1] = buf[(j2 + N2 * j1) * W + w];
+    for (int j1 = 0; j1 < N1; j1++) {
+      s[j1] = buf[(j2 + N2 * j1) * W + w];
+      if (pre) s[j1] = cscale(s[j1], pre[j2 + N2 * j1]);
+    }
+    if (scaled) {
+#pragma unroll
+      for (int j1 = 0; j1 < N1; j1++) s[j1] = kscale(s[j1], scale);
+    }
     dft<N1, DIR, N>(s, tw);
 #pragma unroll
     for (int k1 = 1; k1 < N1; k1++) s[k1] = twmul<DIR, N>(s[k1], tw, j2 * k1);
@@ -1000,24 +1010,14 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
         linev[m] = CR(lapl_value(g, ix, iy, iz, a.lap_factor, a.gc));
       }
     } else if constexpr (base_var(VAR) == INV_FINAL || VAR == FWD_VPSI) {
-      for (int m = threadIdx.x; m < N; m += NT)
-        linev[m] = CR(a.V[(pbase + m * g.sp) * a.nspin + a.spin]) + CR(a.vshift);
-    }
-    if constexpr (VAR == FWD_VPSI) {
-      csync<NT>();
-      if (a.nl_offs) {
-        // Fourier-form operator: (V + shift) psi + nonlocal(psi) formed in shared memory before the transform
-        for (int e = threadIdx.x; e < TILE; e += NT) {
-          const int m = e / W, w = e % W, s = s0 + w;
-          if (s < a.S) {
-            const long long pt = pbase + m * g.sp;
-            T v = conv<T>(cscale(conv<TC>(buf[e]), linev[m]));
-            buf[e] = cadd(v, nl_term<R>(a, pt, s));
-          }
-        }
-        csync<NT>();
+      for (int m = threadIdx.x; m < N; m += NT) {
+        const long long pt = pbase + m * g.sp;
+        // Fourier form: points with sphere hits already hold (V + shift) psi + nonlocal
+        const bool masked = VAR == FWD_VPSI && a.nl_offs && a.nl_offs[pt + 1] > a.nl_offs[pt];
+        linev[m] = masked ? CR(1) : CR(a.V[pt * a.nspin + a.spin]) + CR(a.vshift);
       }
     }
+    if constexpr (VAR == FWD_VPSI) csync<NT>();  // the transform's first step reads the factors
 
     // final value of one output element: scaling, epilogue term, Horner step (base + c * value, the
     // value rounded to the storage type first, as the operator's output would be)
@@ -1036,7 +1036,7 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
       return conv<T>(v);
     };
     auto put_out = [&](int m, int w, TC v) { buf[m * W + w] = epi_out(m, w, v); };
-    const CR *pre = (VAR == FWD_VPSI && !a.nl_offs) ? linev : nullptr;
+    const CR *pre = VAR == FWD_VPSI ? linev : nullptr;  // per-point factors of the input
     constexpr int D = dir_first<VAR>();
     const T *twt = reinterpret_cast<const T *>(tw);
 
@@ -1049,12 +1049,6 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
         tile_dft<N, D, W, NT, false, TC>(buf, exch, tw, pre, put_out);
       }
     } else {
-      if constexpr (VAR == FWD_VPSI) {
-        if (!a.nl_offs) {
-          for (int e = threadIdx.x; e < TILE; e += NT) buf[e] = cscale(buf[e], linev[e / W]);
-          csync<NT>();
-        }
-      }
       // plain passes (no scaling, no accumulators) store the transform's values as they are
       const bool plain = !AUX && !scaled;
       if constexpr (VAR == MID_KIN) {
@@ -1072,10 +1066,10 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
       } else if constexpr (AUX) {
         // the epilogue (V psi or the Laplacian term, Taylor accumulators) in the transform's last step
         tile_dft_inplace<N, D, W, NT, T>(buf, twt, epi_out);
-      } else if (VAR == INV_STORE && scaled) {
-        tile_dft_inplace<N, D, W, NT, T>(buf, twt, [&](int, int, T v) { return kscale(v, a.scale); });
+      } else if constexpr (VAR == INV_STORE) {
+        tile_dft_inplace<N, D, W, NT, T>(buf, twt, Identity(), nullptr, scaled, a.scale);
       } else {
-        tile_dft_inplace<N, D, W, NT, T>(buf, twt, Identity());
+        tile_dft_inplace<N, D, W, NT, T>(buf, twt, Identity(), pre);
         if (!plain) {
           csync<NT>();
           for (int e = threadIdx.x; e < TILE; e += NT) put_out(e / W, e % W, buf[e]);
@@ -1582,13 +1576,14 @@ void launch_zlines(Ctx &ctx, const Basis &b, const PassArgs<R> &a, const ZLines 
 
 template <typename R, int N>
 void launch_n(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg, int var) {
-  if (gg.axis == 2 && var != FWD_VPSI && (sizeof(R) == 8 || single_arith(ctx, a, var))) {
+  if (gg.axis == 2 && (sizeof(R) == 8 || single_arith(ctx, a, var))) {
     const ZLines z = zlines_of(ctx, b, a.S, int(sizeof(C2<R>)));
     if (z.lpt > 0) {
       switch (var) {
         case FWD_STORE: launch_zlines<R, N, FWD_STORE>(ctx, b, a, z); return;
         case INV_STORE: launch_zlines<R, N, INV_STORE>(ctx, b, a, z); return;
         case INV_FINAL: launch_zlines<R, N, INV_FINAL>(ctx, b, a, z); return;
+        case FWD_VPSI: launch_zlines<R, N, FWD_VPSI>(ctx, b, a, z); return;
         case FWD_PERM: launch_zlines<R, N, FWD_PERM>(ctx, b, a, z); return;
         case INV_PERM: launch_zlines<R, N, INV_PERM>(ctx, b, a, z); return;
         case INV_FINAL_PERM: launch_zlines<R, N, INV_FINAL_PERM>(ctx, b, a, z); return;
@@ -1638,7 +1633,7 @@ template <typename R> bool launch(Ctx &ctx, const Basis &b, const PassArgs<R> &a
   // y and x passes over flattened columns (their second input, the Laplacian term's, lies alike)
   const bool flat = flat_ok(ctx, b, a.S, int(sizeof(T)), a.axis) &&
                     (var == FWD_STORE || var == INV_STORE || var == MID_KIN || var == FWD_LAPLADD);
-  const bool zl = a.axis == 2 && same_type && var != FWD_VPSI && zlines_of(ctx, b, a.S, int(sizeof(T))).lpt > 0;
+  const bool zl = a.axis == 2 && same_type && zlines_of(ctx, b, a.S, int(sizeof(T))).lpt > 0;
   if (!flat && !zl) {
     if (a.S < 256 / int(sizeof(T))) return false;  // fewer states than one 256-byte row: generic kernel
     // rows that are not 16-byte multiples (an odd number of single-precision states): only the kernels with

@@ -1,5 +1,5 @@
 // Device pieces shared by the FFT pass kernels (fft.cu, fft2.cuh): radix codelets,
-// line geometry, the Laplacian factor and the per-point nonlocal term.
+// line geometry and the Laplacian factor.
 #pragma once
 
 #include "inqb_internal.h"
@@ -195,24 +195,6 @@ __device__ __forceinline__ double lapl_value(const Geom &g, int ix, int iy, int 
   double c2 = (g.rlat[0][2] * G0 + g.rlat[1][2] * G1) + g.rlat[2][2] * G2;
   double g2 = c0 * c0 + c1 * c1 + c2 * c2;
   return factor * (-g2 + (gc[0] * G0 + gc[1] * G1 + gc[2] * G2));
-}
-
-// nonlocal term at one grid point and state: sum over sphere hits h of sum_l hcoef[h][l] * projD[p][l][s]
-template <typename R>
-__device__ __forceinline__ C2<R> nl_term(const PassArgs<R> &a, long long pt, int s) {
-  using T = C2<R>;
-  T acc = mk<T>(R(0), R(0));
-  const int h0 = __ldg(&a.nl_offs[pt]), h1 = __ldg(&a.nl_offs[pt + 1]);
-  for (int h = h0; h < h1; h++) {
-    const int p = __ldg(&a.nl_hitp[h]);
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-      T c = a.nl_hcoef[h * 4 + l];
-      T pj = a.projD[((long long)p * 4 + l) * a.S + s];
-      acc = cadd(acc, cmul(c, pj));
-    }
-  }
-  return acc;
 }
 
 }  // namespace inqb

@@ -209,10 +209,7 @@ template <typename R> struct PassArgs {
   const R *V = nullptr;
   int nspin = 1, spin = 0;
   R vshift = R(0);
-  const int *nl_offs = nullptr;
-  const int *nl_hitp = nullptr;     // projector index of each hit
-  const C2<R> *nl_hcoef = nullptr;
-  const C2<R> *projD = nullptr;
+  const int *nl_offs = nullptr;     // prologue: sphere hits per point; points that have some are not multiplied by V
   // Horner step of a Taylor exponential (real-space final pass): out = hbase + hc * (H v), where v is
   // the pass's orbital input; hbase may not alias `out` (the operator's intermediates live there)
   const C2<R> *hbase = nullptr;
@@ -233,9 +230,11 @@ void launch_nl_project(Ctx &ctx, const Basis &b, const Hamiltonian &h, const C2<
 void launch_nl_tables(Ctx &ctx, const Basis &b, Hamiltonian &h, const double kA[3]);
 template <typename R>
 void launch_nl_scatter(Ctx &ctx, const Basis &b, const Hamiltonian &h, const C2<R> *projD, int S, C2<R> *out);
-// out += term (scaled: out += scale * term) at the sphere points
+// out += term (scaled: out += scale * term) at the sphere points; with V (nspin, spin, vshift) given,
+// out = (V + vshift) out + term there
 template <typename R>
-void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, C2<R> *out, bool scaled, C2<R> scale);
+void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, C2<R> *out, bool scaled, C2<R> scale,
+                     const R *V = nullptr, int nspin = 1, int spin = 0, R vshift = R(0));
 // Taylor terms combined: e1 = x + sum_n c1[n] u[n], e2 = x + sum_n c2[n] u[n] (n < nterms <= 8, summed in
 // order n = 0, 1, ...); e1 may be null, e2 may equal x
 template <typename R>

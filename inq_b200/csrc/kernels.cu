@@ -101,11 +101,11 @@ template <typename T> __device__ __forceinline__ T cmac(T acc, T a, T b) {
 
 // The bulk-copy forms of the projection and the apply run NLA_NT compute threads beside one producer
 // warp that moves whole rows of states (contiguous in the state-fastest layout) with bulk
-// asynchronous copies.  The compute threads synchronise among themselves on named barrier 1.
+// asynchronous copies.  The projection's compute threads synchronise among
+// themselves on named barrier 1.
 constexpr int NLA_NT = 128;
 
-__device__ __forceinline__ void nla_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NLA_NT) : "memory"); }
-// the same barrier, returning whether any compute thread passed a nonzero value (uniform result)
+// that barrier, returning whether any compute thread passed a nonzero value (uniform result)
 __device__ __forceinline__ bool nla_sync_or(int v) {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
@@ -132,26 +132,30 @@ __device__ __forceinline__ bool nla_wait(uint64_t *b, uint32_t parity, volatile 
 // ------------------------------------------------------------------ nonlocal projection
 // proj[p][l][s] = sum_i gcoef[p][i][l] * psi[pt_i][s]; projD = coeff[p] . proj
 // (projector_all.hpp:113-211).  Stage 1: CTA = (projector p, range rg of its sphere points, chunk of
-// 32 K states); each of its 8 warps takes a contiguous run of the range, reads 32 point indices with
-// one coalesced load and hands them out by shuffles, and keeps NP points in flight; a lane holds K
-// states 32 apart, so each point costs K contiguous 256-byte segments of the state-fastest row.  The
-// warp partials are summed in order into partial[p][rg][l][s].  Stage 2 sums the ranges in order and
-// applies the KB coefficients.
+// K << sl states); each of its 8 warps takes a contiguous run of the range, reads 32 point indices with
+// one coalesced load and hands them out by shuffles, and keeps NP points per lane group in flight.  A group
+// of 2^sl lanes holds K states each, 2^sl apart; sets of at most 32 states use groups of as many lanes as
+// they have states (a power of two), so that a warp takes several points at a time instead of idling its
+// lanes.  Groups are summed by shuffles in a fixed tree, the warps in order into partial[p][rg][l][s].
+// Stage 2 sums the ranges in order and applies the KB coefficients.  Latency-bound (a chain of index, row
+// and coefficient loads per batch): what counts is few batches per warp.
 constexpr int NLP_WARPS = 8, NLP_RANGES = 16;  // 16 ranges: the bulk projection 181 us against 218 with 8 (FP64, 96^3 x 256)
+constexpr int NLP_MAX_RANGES = 32;
 
-template <typename R, typename A, int K>
-__global__ void __launch_bounds__(NLP_WARPS * 32) nl_project_kernel(const C2<R> *__restrict__ psi, int S,
+template <typename R, typename A, int K, int NP>
+__global__ void __launch_bounds__(NLP_WARPS * 32) nl_project_kernel(const C2<R> *__restrict__ psi, int S, int sl,
                                                                     const int *__restrict__ pt,
                                                                     const C2<A> *__restrict__ gcoef,
                                                                     const int *__restrict__ npts, int maxsph,
                                                                     C2<A> *__restrict__ partial) {
   using T = C2<R>;
   using TA = C2<A>;
-  constexpr int NP = 4;  // points in flight per warp
   __shared__ TA part[NLP_WARPS][4][32 * K];
   const int p = blockIdx.x, rg = blockIdx.y;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  const int sbase = blockIdx.z * 32 * K;
+  const int SL = 1 << sl, G = 32 >> sl;        // lanes per group, groups per warp
+  const int ls = lane & (SL - 1), g = lane >> sl;
+  const int sbase = blockIdx.z * SL * K;
   const int np = npts[p];
   const int nr = int(gridDim.y);  // ranges of a sphere
   const int rper = (np + nr - 1) / nr;
@@ -167,24 +171,26 @@ __global__ void __launch_bounds__(NLP_WARPS * 32) nl_project_kernel(const C2<R> 
   for (int base = i0; base < i1; base += 32) {
     const int cnt = min(32, i1 - base);
     const int qv = lane < cnt ? __ldg(&pt[rowbase + base + lane]) : 0;
-    for (int j = 0; j < cnt; j += NP) {
+    for (int j = 0; j < cnt; j += NP * G) {
       T x[NP][K];
 #pragma unroll
       for (int u = 0; u < NP; u++) {
-        const long long q = __shfl_sync(0xffffffffu, qv, (j + u) & 31);
+        const int i = j + u * G + g;
+        const long long q = __shfl_sync(0xffffffffu, qv, i & 31);
 #pragma unroll
         for (int k = 0; k < K; k++) {
-          const int s = sbase + k * 32 + lane;
-          x[u][k] = (j + u < cnt && s < S) ? psi[q * S + s] : mk<T>(R(0), R(0));
+          const int s = sbase + k * SL + ls;
+          x[u][k] = (i < cnt && s < S) ? psi[q * S + s] : mk<T>(R(0), R(0));
         }
       }
 #pragma unroll
       for (int u = 0; u < NP; u++) {
-        if (j + u < cnt) {
-          const TA *g = gcoef + (rowbase + base + j + u) * 4;
+        const int i = j + u * G + g;
+        if (i < cnt) {
+          const TA *gc = gcoef + (rowbase + base + i) * 4;
           TA gl[4];
 #pragma unroll
-          for (int l = 0; l < 4; l++) gl[l] = g[l];
+          for (int l = 0; l < 4; l++) gl[l] = gc[l];
 #pragma unroll
           for (int k = 0; k < K; k++) {
             const TA v = mk<TA>(A(x[u][k].x), A(x[u][k].y));
@@ -198,13 +204,19 @@ __global__ void __launch_bounds__(NLP_WARPS * 32) nl_project_kernel(const C2<R> 
 #pragma unroll
   for (int k = 0; k < K; k++)
 #pragma unroll
-    for (int l = 0; l < 4; l++) part[wp][l][k * 32 + lane] = acc[k][l];
+    for (int l = 0; l < 4; l++) {
+      for (int o = 16; o >= SL; o >>= 1) {
+        acc[k][l].x += __shfl_down_sync(0xffffffffu, acc[k][l].x, o);
+        acc[k][l].y += __shfl_down_sync(0xffffffffu, acc[k][l].y, o);
+      }
+      if (g == 0) part[wp][l][k * SL + ls] = acc[k][l];
+    }
   __syncthreads();
-  for (int e = threadIdx.x; e < 4 * 32 * K; e += blockDim.x) {
-    const int l = e / (32 * K), sl = e % (32 * K);
-    const int s = sbase + sl;
-    TA t = part[0][l][sl];
-    for (int w = 1; w < NLP_WARPS; w++) t = cadd(t, part[w][l][sl]);
+  for (int e = threadIdx.x; e < 4 * SL * K; e += blockDim.x) {
+    const int l = e / (SL * K), c = e % (SL * K);
+    const int s = sbase + c;
+    TA t = part[0][l][c];
+    for (int w = 1; w < NLP_WARPS; w++) t = cadd(t, part[w][l][c]);
     if (s < S) partial[(((long long)p * nr + rg) * 4 + l) * S + s] = t;
   }
 }
@@ -339,29 +351,46 @@ __global__ void __launch_bounds__(NLA_NT + 32) nl_project_bulk_kernel(const C2<R
   }
 }
 
+// Block = 32 states x 4 functions of one projector: a thread sums its function's ranges in order, eight
+// loads in flight (one thread per projector and state, with a load at a time, took 10 us at any size).
+constexpr int NLF_S = 32;
+
 template <typename R, typename A>
-__global__ void nl_project_finish_kernel(const C2<A> *__restrict__ partial, int nproj, int nr, int S,
-                                         const A *__restrict__ coeff, C2<R> *projraw, C2<R> *projD) {
+__global__ void __launch_bounds__(NLF_S * 4) nl_project_finish_kernel(const C2<A> *__restrict__ partial, int nsb, int nr,
+                                                                      int S, const A *__restrict__ coeff,
+                                                                      C2<R> *projraw, C2<R> *projD) {
   using T = C2<R>;
   using TA = C2<A>;
-  const long long n = (long long)nproj * S;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int p = int(e / S), s = int(e % S);
-    TA pr[4];
+  __shared__ TA pr[4][NLF_S];
+  const int p = blockIdx.x / nsb, l = threadIdx.x / NLF_S, c = threadIdx.x % NLF_S;
+  const int s = (blockIdx.x % nsb) * NLF_S + c;
+  if (s < S) {
+    const TA *src = partial + ((long long)p * nr * 4 + l) * S + s;
+    const long long step = 4LL * S;
+    TA t = src[0];
+    int rg = 1;
+    for (; rg + 8 <= nr; rg += 8) {
+      TA v[8];
 #pragma unroll
-    for (int l = 0; l < 4; l++) {
-      TA t = partial[(((long long)p * nr) * 4 + l) * S + s];
-      for (int rg = 1; rg < nr; rg++) t = cadd(t, partial[(((long long)p * nr + rg) * 4 + l) * S + s]);
-      pr[l] = t;
-      projraw[((long long)p * 4 + l) * S + s] = mk<T>(R(t.x), R(t.y));
+      for (int u = 0; u < 8; u++) v[u] = src[(rg + u) * step];
+#pragma unroll
+      for (int u = 0; u < 8; u++) t = cadd(t, v[u]);
     }
+    TA v[7];
 #pragma unroll
-    for (int l = 0; l < 4; l++) {
-      TA t = mk<TA>(A(0), A(0));
+    for (int u = 0; u < 7; u++) v[u] = rg + u < nr ? src[(rg + u) * step] : mk<TA>(A(0), A(0));
 #pragma unroll
-      for (int j = 0; j < 4; j++) t = cadd(t, cscale(pr[j], coeff[(p * 4 + l) * 4 + j]));
-      projD[((long long)p * 4 + l) * S + s] = mk<T>(R(t.x), R(t.y));
-    }
+    for (int u = 0; u < 7; u++)
+      if (rg + u < nr) t = cadd(t, v[u]);
+    pr[l][c] = t;
+    projraw[((long long)p * 4 + l) * S + s] = mk<T>(R(t.x), R(t.y));
+  }
+  __syncthreads();
+  if (s < S) {
+    TA t = mk<TA>(A(0), A(0));
+#pragma unroll
+    for (int j = 0; j < 4; j++) t = cadd(t, cscale(pr[j][c], coeff[(p * 4 + l) * 4 + j]));
+    projD[((long long)p * 4 + l) * S + s] = mk<T>(R(t.x), R(t.y));
   }
 }
 
@@ -372,71 +401,71 @@ void launch_nl_project(Ctx &ctx, const Basis &b, const Hamiltonian &h, const C2<
   if (P.nproj == 0) return;
   const bool dbl = sizeof(R) == 8 || ctx.mixed_compute != 0;  // double-precision coefficients and sums
   // ranges per sphere (option nl_project_ranges; the summation order follows it)
-  const int NR = ctx.nl_project_ranges > 0 ? ctx.nl_project_ranges : NLP_RANGES;
-  const size_t pbytes = size_t(P.nproj) * NR * 4 * S * (dbl ? sizeof(double2) : sizeof(float2));
-  void *partial = dev_alloc(ctx, pbytes);
-  const long long fin = (long long)P.nproj * S;
-  // bulk form: rows of 16-byte multiples, and (automatic choice) enough CTAs to fill the device; the
-  // choice (and so the summation order) follows the device's SM count, not the grid_sms option
+  int NR = ctx.nl_project_ranges > 0 ? ctx.nl_project_ranges : NLP_RANGES;
+  // bulk form: rows of 16-byte multiples, and (automatic choice) more than 32 states and, with at most 32
+  // ranges, two CTAs per SM; the choice (and so the summation order) follows the device's SM count, not the
+  // grid_sms option.  Fewer states leave most of the bulk form's threads idle: 8 states of 24 projectors
+  // 29 us against 9 in the register form; 50 FP64 states of 12 projectors 19 against 28.
   constexpr int JB = 2;
   const size_t row_bytes = size_t(S) * sizeof(C2<R>);
   const int nchunks = (S + NLA_NT * JB - 1) / (NLA_NT * JB);
   const bool bulk_ok = row_bytes % 16 == 0 && reinterpret_cast<uintptr_t>(psi) % 16 == 0;
   const bool bulk = bulk_ok && (ctx.nl_bulk > 0 ||
-                                (ctx.nl_bulk == 0 && (long long)P.nproj * NR * nchunks >= 2LL * ctx.device_sms));
-  if (bulk) {
-    const int SCmax = std::min(NLA_NT * JB, S);
-    const size_t srow = size_t(SCmax) * sizeof(C2<R>);
-    int KB = ctx.nl_project_points > 0 ? ctx.nl_project_points : int(16384 / srow);  // about 16 KB of rows per stage
-    KB = KB < 1 ? 1 : (KB > 32 ? 32 : KB);
-    const size_t abytes = dbl ? sizeof(double2) : sizeof(float2);
-    auto smem_of = [&](int kb) {
-      return size_t(NLP_NS) * kb * srow + size_t(NLP_NS) * kb * 4 * abytes + 2 * NLP_NS * sizeof(uint64_t) + 16;
-    };
-    while (KB > 1 && smem_of(KB) > size_t(ctx.max_smem_optin)) KB--;  // an option asking for more than fits
-    const size_t smem = smem_of(KB);
-    const dim3 grid(P.nproj, NR, nchunks);
-    if (dbl) {
-      auto kern = nl_project_bulk_kernel<R, double, JB>;
+                                (ctx.nl_bulk == 0 && S > 32 &&
+                                 (long long)P.nproj * std::max(NR, NLP_MAX_RANGES) * nchunks >= 2LL * ctx.device_sms));
+  // register form: two states per lane, or one in lane groups of a power of two
+  int sl = 5, K = 2;
+  if (S <= 32) {
+    K = 1;
+    for (sl = 0; (1 << sl) < S; sl++) {
+    }
+  }
+  const int rchunks = (S + (K << sl) - 1) / (K << sl);
+  // few projectors: more, shorter ranges until the device has two CTAs per SM (8 projectors of 16 FP64 states:
+  // projection and finish 10.7 us with 16 ranges, 9.4 with 32, 13.7 with 64)
+  if (ctx.nl_project_ranges == 0)
+    while (NR < NLP_MAX_RANGES && (long long)P.nproj * NR * (bulk ? nchunks : rchunks) < 2LL * ctx.device_sms) NR *= 2;
+  void *partial = dev_alloc(ctx, size_t(P.nproj) * NR * 4 * S * (dbl ? sizeof(double2) : sizeof(float2)));
+  auto go = [&](auto atype) {
+    using A = decltype(atype);
+    using TA = C2<A>;
+    const TA *gcoef;
+    const A *coeff;
+    if constexpr (sizeof(A) == 8) gcoef = P.d_gcoef, coeff = P.d_coeff;
+    else gcoef = P.d_gcoef32, coeff = P.d_coeff32;
+    TA *part = static_cast<TA *>(partial);
+    if (bulk) {
+      const int SCmax = std::min(NLA_NT * JB, S);
+      const size_t srow = size_t(SCmax) * sizeof(C2<R>);
+      int KB = ctx.nl_project_points > 0 ? ctx.nl_project_points : int(16384 / srow);  // about 16 KB of rows per stage
+      KB = KB < 1 ? 1 : (KB > 32 ? 32 : KB);
+      auto smem_of = [&](int kb) {
+        return size_t(NLP_NS) * kb * srow + size_t(NLP_NS) * kb * 4 * sizeof(TA) + 2 * NLP_NS * sizeof(uint64_t) + 16;
+      };
+      while (KB > 1 && smem_of(KB) > size_t(ctx.max_smem_optin)) KB--;  // an option asking for more than fits
+      const size_t smem = smem_of(KB);
+      auto kern = nl_project_bulk_kernel<R, A, JB>;
       ensure_smem_attr(reinterpret_cast<const void *>(kern), smem);
-      kern<<<grid, NLA_NT + 32, smem, ctx.stream>>>(psi, S, P.d_pt, P.d_gcoef, P.d_npts, P.maxsph, KB,
-                                                    static_cast<double2 *>(partial), ctx.d_err);
-      LAUNCHED(ctx);
-      nl_project_finish_kernel<R, double><<<grid_for(fin, 256), 256, 0, ctx.stream>>>(
-          static_cast<const double2 *>(partial), P.nproj, NR, S, P.d_coeff, projraw, projD);
+      kern<<<dim3(P.nproj, NR, nchunks), NLA_NT + 32, smem, ctx.stream>>>(psi, S, P.d_pt, gcoef, P.d_npts, P.maxsph, KB,
+                                                                        part, ctx.d_err);
     } else {
-      auto kern = nl_project_bulk_kernel<R, float, JB>;
-      ensure_smem_attr(reinterpret_cast<const void *>(kern), smem);
-      kern<<<grid, NLA_NT + 32, smem, ctx.stream>>>(psi, S, P.d_pt, P.d_gcoef32, P.d_npts, P.maxsph, KB,
-                                                    static_cast<float2 *>(partial), ctx.d_err);
-      LAUNCHED(ctx);
-      nl_project_finish_kernel<R, float><<<grid_for(fin, 256), 256, 0, ctx.stream>>>(
-          static_cast<const float2 *>(partial), P.nproj, NR, S, P.d_coeff32, projraw, projD);
+      const dim3 grid(P.nproj, NR, rchunks);
+      // four points in flight at two states per lane (eight: 94 against 50 us at 72^3 x 99 single)
+      if (K == 2)
+        nl_project_kernel<R, A, 2, 4><<<grid, NLP_WARPS * 32, 0, ctx.stream>>>(psi, S, sl, P.d_pt, gcoef, P.d_npts,
+                                                                                P.maxsph, part);
+      else
+        nl_project_kernel<R, A, 1, 8><<<grid, NLP_WARPS * 32, 0, ctx.stream>>>(psi, S, sl, P.d_pt, gcoef, P.d_npts,
+                                                                              P.maxsph, part);
     }
     LAUNCHED(ctx);
-    dev_free(ctx, partial);
-    return;
-  }
-  if (dbl) {
-    constexpr int K = 2;
-    dim3 grid(P.nproj, NR, (S + 32 * K - 1) / (32 * K));
-    nl_project_kernel<R, double, K><<<grid, NLP_WARPS * 32, 0, ctx.stream>>>(
-        psi, S, P.d_pt, P.d_gcoef, P.d_npts, P.maxsph, static_cast<double2 *>(partial));
+    const int nsb = (S + NLF_S - 1) / NLF_S;
+    nl_project_finish_kernel<R, A><<<unsigned(P.nproj) * nsb, NLF_S * 4, 0, ctx.stream>>>(part, nsb, NR, S, coeff,
+                                                                                         projraw, projD);
     LAUNCHED(ctx);
-    nl_project_finish_kernel<R, double><<<grid_for(fin, 256), 256, 0, ctx.stream>>>(
-        static_cast<const double2 *>(partial), P.nproj, NR, S, P.d_coeff, projraw, projD);
-  } else {
-    // two states per lane (64-state chunks) in single precision too: more CTAs with fewer registers
-    // hide the gather latency better (measured 168 us against 202 us with four at 96^3 x 256)
-    constexpr int K = 2;
-    dim3 grid(P.nproj, NR, (S + 32 * K - 1) / (32 * K));
-    nl_project_kernel<R, float, K><<<grid, NLP_WARPS * 32, 0, ctx.stream>>>(
-        psi, S, P.d_pt, P.d_gcoef32, P.d_npts, P.maxsph, static_cast<float2 *>(partial));
-    LAUNCHED(ctx);
-    nl_project_finish_kernel<R, float><<<grid_for(fin, 256), 256, 0, ctx.stream>>>(
-        static_cast<const float2 *>(partial), P.nproj, NR, S, P.d_coeff32, projraw, projD);
-  }
-  LAUNCHED(ctx);
+  };
+  if (dbl) go(double());
+  else go(float());
   dev_free(ctx, partial);
 }
 
@@ -474,94 +503,115 @@ void launch_nl_scatter(Ctx &ctx, const Basis &b, const Hamiltonian &h, const C2<
 
 // out[pt][s] += nonlocal term at the grid points that lie in a sphere (ks_hamiltonian.hpp:153,
 // projector_all.hpp:276-288), hits of a point summed in projector order, no atomics; optionally scaled,
-// out += scale * term (a Horner step of a Taylor exponential).
-// Owner computes: one warp per (grid point with sphere hits, chunk of 32 * U states), lanes over states.
-// The point's record gives its first hit and projector in one load, so the coefficient, projection and
-// output reads are all issued together (a two-level dependency instead of point -> CSR -> hit ->
-// projection); splitting the states into chunks keeps the registers low and many warps resident.
-template <typename R>
-__global__ void __launch_bounds__(128) nl_apply_kernel(long long nitems, int nchunks, int S,
-                                                          const int4 *__restrict__ hrec, const int *__restrict__ hitp,
-                                                          const C2<R> *__restrict__ hcoef,
-                                                          const C2<R> *__restrict__ projD, C2<R> *__restrict__ out,
-                                                          bool scaled, C2<R> scale) {
+// out += scale * term (a Horner step of a Taylor exponential), or with the local potential,
+// out = (V + vshift) out + term (the Fourier form, whose next pass multiplies the other points by it).
+template <typename R> struct NlApply {
+  const int4 *hrec;
+  const int *hitp;
+  const C2<R> *hcoef;
+  const C2<R> *projD;
+  C2<R> *out;
+  int S;
+  bool scaled;
+  C2<R> scale;
+  const R *V;  // null: out += term
+  int nspin, spin;
+  R vshift;
+};
+// the term's first hit is summed by the caller (fused products); the others follow
+// (VM: with the local potential; a runtime choice cost 177 against 155 us at 96^3 x 256 single)
+template <typename R, bool VM>
+__device__ __forceinline__ C2<R> nl_value(const NlApply<R> &a, long long pt, int s, int h0, int nh, C2<R> o,
+                                          const C2<R> (&hc)[4], const C2<R> (&pd)[4]) {
   using T = C2<R>;
-  constexpr int U = 16 / sizeof(R);  // states per lane: 4 single, 2 double
-  const int lane = threadIdx.x & 31;
-  const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  // the record of the warp's next item is requested while the current one is processed
-  int4 next = warp < nitems ? hrec[warp / nchunks] : make_int4(0, 0, 0, 0);
-  for (long long it = warp; it < nitems; it += nwarps) {
-    const int s0 = int(it % nchunks) * (32 * U);
+  T accv = mk<T>(R(0), R(0));
+#pragma unroll
+  for (int l = 0; l < 4; l++) accv = cmac(accv, hc[l], pd[l]);
+#pragma unroll 1  // few points lie in more than one sphere: no registers for them
+  for (int k = 1; k < nh; k++) {
+    const int h = h0 + k;
+    const int p = a.hitp[h];
+#pragma unroll
+    for (int l = 0; l < 4; l++)
+      accv = cadd(accv, cmul(a.hcoef[(long long)h * 4 + l], a.projD[((long long)p * 4 + l) * a.S + s]));
+  }
+  if constexpr (VM) o = cscale(o, a.V[pt * a.nspin + a.spin] + a.vshift);
+  return cadd(o, a.scaled ? cmul(a.scale, accv) : accv);
+}
+
+// Register form.  Owner computes: one group of 2^sl lanes per (grid point with sphere hits, chunk of
+// U << sl states), lanes over states.  The point's record gives its first hit and projector in one load, so
+// the coefficient, projection and output reads are all issued together (a two-level dependency instead of
+// point -> CSR -> hit -> projection); splitting the states into chunks keeps the registers low and many
+// warps resident.
+template <typename R, int U, bool VM>
+__global__ void __launch_bounds__(128) nl_apply_kernel(NlApply<R> a, long long nitems, int nchunks, int sl) {
+  using T = C2<R>;
+  const int S = a.S, SL = 1 << sl;
+  const int ls = threadIdx.x & (SL - 1);
+  const long long group = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> sl;
+  const long long ngroups = ((long long)gridDim.x * blockDim.x) >> sl;
+  // the record of the group's next item is requested while the current one is processed
+  int4 next = group < nitems ? a.hrec[group / nchunks] : make_int4(0, 0, 0, 0);
+  for (long long it = group; it < nitems; it += ngroups) {
+    const int s0 = int(it % nchunks) * (SL * U);
     const int4 rec = next;
-    if (it + nwarps < nitems) next = hrec[(it + nwarps) / nchunks];
+    if (it + ngroups < nitems) next = a.hrec[(it + ngroups) / nchunks];
     const long long pt = rec.x;
     const int h0 = rec.y, nh = rec.z, p0 = rec.w;
-    T hc[4], o[U], pd[4][U];
+    T hc[4], o[U], pd[U][4];
 #pragma unroll
-    for (int l = 0; l < 4; l++) hc[l] = hcoef[(long long)h0 * 4 + l];
+    for (int l = 0; l < 4; l++) hc[l] = a.hcoef[(long long)h0 * 4 + l];
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const int s = s0 + u * 32 + lane;
+      const int s = s0 + u * SL + ls;
       if (s < S) {
-        o[u] = out[pt * S + s];
+        o[u] = a.out[pt * S + s];
 #pragma unroll
-        for (int l = 0; l < 4; l++) pd[l][u] = projD[((long long)p0 * 4 + l) * S + s];
+        for (int l = 0; l < 4; l++) pd[u][l] = a.projD[((long long)p0 * 4 + l) * S + s];
       }
     }
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const int s = s0 + u * 32 + lane;
-      if (s >= S) continue;
-      T accv = mk<T>(R(0), R(0));
-#pragma unroll
-      for (int l = 0; l < 4; l++) accv = cadd(accv, cmul(hc[l], pd[l][u]));
-      for (int k = 1; k < nh; k++) {
-        const int h = h0 + k;
-        const int p = hitp[h];
-#pragma unroll
-        for (int l = 0; l < 4; l++)
-          accv = cadd(accv, cmul(hcoef[(long long)h * 4 + l], projD[((long long)p * 4 + l) * S + s]));
-      }
-      const long long e = pt * S + s;
-      out[e] = cadd(o[u], scaled ? cmul(scale, accv) : accv);
+      const int s = s0 + u * SL + ls;
+      if (s < S) a.out[pt * S + s] = nl_value<R, VM>(a, pt, s, h0, nh, o[u], hc, pd[u]);
     }
   }
 }
 
-// Bulk-copy form of the apply.  A CTA takes batches of KB consecutive hit points: a producer warp
-// copies the points' output rows (S contiguous states each) into shared memory with bulk asynchronous
-// copies, the compute threads add the nonlocal term to them there, and the producer writes the rows
-// back with bulk copies.  Two stages overlap one batch's copies with the next batch's arithmetic, and
-// the copy engine keeps the bytes in flight that the register-held form could not.  The terms are
-// summed in nl_apply_kernel's order, with fused multiply-adds (single precision: 0.19 against 0.20 ms
-// at 96^3 x 256, and six CTAs per SM, 0.18 ms; double: 0.31 against 0.32 ms).
+// Bulk-copy form of the apply.  A CTA takes batches of KB consecutive hit points: a producer warp copies
+// the points' output rows (S contiguous states each) into shared memory with bulk asynchronous copies, two
+// batches ahead, so the copy engine keeps the bytes in flight that the register form cannot; the compute
+// threads, in groups of 2^ts per row, add the nonlocal term and store the rows to global memory, or with BS
+// to shared memory, from where bulk copies take them (rows of 2 KB single, where the stores are many: 151
+// against 207 us at 96^3 x 256; no difference for shorter rows and double).  Rows that are not 16-byte
+// multiples (odd single-precision counts) are copied with the 8 bytes before or after them, up to 16-byte
+// boundaries; only their own states are stored.  The terms are summed in nl_apply_kernel's order.  Bound by
+// HBM: 2 S elements per hit point; 120^3 x 64 FP64 328 -> 163 us, 32^3 x 16 FP64 23 -> 8.6 us against a
+// thread per state and batches of 8 points.
 constexpr int NLA_NS = 2;     // stages
 constexpr int NLA_KMAX = 32;  // largest batch (one producer lane per row)
 
-template <typename R, int J>
-__global__ void __launch_bounds__(NLA_NT + 32, sizeof(R) == 4 ? 6 : 3) nl_apply_bulk_kernel(long long nrec, int KB, int S,
-                                                                     const int4 *__restrict__ hrec,
-                                                                     const int *__restrict__ hitp,
-                                                                     const C2<R> *__restrict__ hcoef,
-                                                                     const C2<R> *__restrict__ projD, C2<R> *out,
-                                                                     bool scaled, C2<R> scale, int *err) {
+template <typename R, int J, bool BS, bool VM>
+__global__ void __launch_bounds__(NLA_NT + 32, sizeof(R) == 4 ? 6 : 3) nl_apply_bulk_kernel(NlApply<R> a, long long nrec,
+                                                                                         int KB, int ts, int *err) {
   using T = C2<R>;
   using namespace ptx;
   extern __shared__ __align__(128) unsigned char smem[];
-  T *rows = reinterpret_cast<T *>(smem);                                 // [NS][KB][S]
-  T *hcs = rows + size_t(NLA_NS) * KB * S;                               // [KB][4] first-hit coefficients
-  int4 *recs = reinterpret_cast<int4 *>(hcs + NLA_KMAX * 4);             // [NS][KMAX]
-  uint64_t *full = reinterpret_cast<uint64_t *>(recs + NLA_NS * NLA_KMAX);  // rows and records loaded
+  const int S = a.S;
+  const uint32_t row_bytes = uint32_t(S) * uint32_t(sizeof(T));
+  const uint32_t slot = (row_bytes + 15) & ~15u;                         // bytes copied per row
+  unsigned char *rows = smem;                                            // [NS][KB][slot]
+  T *coefs = reinterpret_cast<T *>(rows + size_t(NLA_NS) * KB * slot);   // [NS][KB][4]
+  int4 *recs = reinterpret_cast<int4 *>(coefs + NLA_NS * KB * 4);        // [NS][KB]
+  uint64_t *full = reinterpret_cast<uint64_t *>(recs + NLA_NS * KB);     // rows, coefficients and records loaded
   uint64_t *done = full + NLA_NS;                                        // rows computed
   volatile int *abort_flag = reinterpret_cast<volatile int *>(done + NLA_NS);
   const long long nbatch = (nrec + KB - 1) / KB;
-  const uint32_t row_bytes = uint32_t(S) * uint32_t(sizeof(T));
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int st = 0; st < NLA_NS; st++) {
-      mbar_init(&full[st], 1);
+      mbar_init(&full[st], 2);
       mbar_init(&done[st], NLA_NT);
     }
     mbar_init_fence();
@@ -570,154 +620,181 @@ __global__ void __launch_bounds__(NLA_NT + 32, sizeof(R) == 4 ? 6 : 3) nl_apply_
   auto wait_bar = [&](uint64_t *b, uint32_t parity) { return nla_wait(b, parity, abort_flag, err); };
 
   if (threadIdx.x >= NLA_NT) {
-    // producer warp: lane q copies row q of a batch in and out
+    // producer warp: lane q copies row q of a batch
     const int lane = threadIdx.x - NLA_NT;
-    auto issue = [&](int st, long long b) {
+    // the k-th batch's stage is computed: with BS its rows are copied out
+    auto retire = [&](int k, long long b) -> bool {
+      const int st = k % NLA_NS;
+      if (!__all_sync(0xffffffffu, wait_bar(&done[st], uint32_t(k / NLA_NS) & 1u))) return false;
+      if constexpr (BS) {
+        const int nb = int(min((long long)KB, nrec - b * KB));
+        if (lane < nb)
+          bulk_store(a.out + (long long)recs[st * KB + lane].x * S, rows + (size_t(st) * KB + lane) * slot, row_bytes);
+        bulk_commit();
+        bulk_wait_read0();  // the stage may be refilled once its rows are read out
+        __syncwarp();
+      }
+      return true;
+    };
+    int k = 0;
+    long long b = blockIdx.x;
+    bool live = true;
+    for (; b < nbatch; b += gridDim.x, k++) {
+      const int st = k % NLA_NS;
       const long long k0 = b * KB;
       const int nb = int(min((long long)KB, nrec - k0));
       int4 rec = make_int4(0, 0, 0, 0);
+      if (lane < nb) rec = a.hrec[k0 + lane];
+      if (k >= NLA_NS && !(live = retire(k - NLA_NS, b - (long long)NLA_NS * gridDim.x))) break;
+      if (lane < nb) recs[st * KB + lane] = rec;
+      if (lane == 0) mbar_expect_tx(&full[st], uint32_t(nb) * slot);
+      __syncwarp();
       if (lane < nb) {
-        rec = hrec[k0 + lane];
-        recs[st * NLA_KMAX + lane] = rec;
+        const uintptr_t src = reinterpret_cast<uintptr_t>(a.out + (long long)rec.x * S) & ~uintptr_t(15);
+        bulk_load(rows + (size_t(st) * KB + lane) * slot, reinterpret_cast<const void *>(src), slot, &full[st]);
+        // the first hit's coefficients by plain loads (bulk copies of 32 bytes: 180 us against 151)
+        const int4 *hc = reinterpret_cast<const int4 *>(a.hcoef + (long long)rec.y * 4);
+        int4 v[4 * sizeof(T) / 16];
+#pragma unroll
+        for (int w = 0; w < int(4 * sizeof(T) / 16); w++) v[w] = __ldg(hc + w);
+#pragma unroll
+        for (int w = 0; w < int(4 * sizeof(T) / 16); w++) reinterpret_cast<int4 *>(coefs + (st * KB + lane) * 4)[w] = v[w];
       }
       __threadfence_block();
       __syncwarp();
-      if (lane == 0) mbar_expect_tx(&full[st], uint32_t(nb) * row_bytes);
-      __syncwarp();
-      if (lane < nb) bulk_load(rows + (size_t(st) * KB + lane) * S, out + (long long)rec.x * S, row_bytes, &full[st]);
-    };
-    int issued = 0;  // batches whose loads were issued, in order
-    for (int st = 0; st < NLA_NS; st++) {
-      const long long b = blockIdx.x + (long long)st * gridDim.x;
-      if (b < nbatch) issue(st, b), issued++;
+      if (lane == 0) mbar_arrive(&full[st]);  // the barrier's second arrival: records and coefficients are there
     }
-    int k = 0;
-    for (long long b = blockIdx.x; b < nbatch; b += gridDim.x, k++) {
-      const int st = k % NLA_NS;
-      if (!wait_bar(&done[st], uint32_t(k / NLA_NS) & 1u)) break;
-      const int nb = int(min((long long)KB, nrec - b * KB));
-      if (lane < nb)
-        bulk_store(out + (long long)recs[st * NLA_KMAX + lane].x * S, rows + (size_t(st) * KB + lane) * S, row_bytes);
-      bulk_commit();
-      bulk_wait_read0();  // the stage may be refilled once its rows are read out
-      __syncwarp();
-      const long long bn = b + (long long)NLA_NS * gridDim.x;
-      if (bn < nbatch) issue(st, bn), issued++;
+    if constexpr (BS) {
+      for (int i = k - NLA_NS < 0 ? 0 : k - NLA_NS; live && i < k; i++)
+        live = retire(i, blockIdx.x + (long long)i * gridDim.x);
+      bulk_wait0();
     }
     // after an abort the compute threads may leave early: wait (bounded) for every issued load to land
     // before the CTA's shared memory is released (on the normal path these phases are already complete)
-    for (int i = issued - NLA_NS < 0 ? 0 : issued - NLA_NS; i < issued; i++)
+    for (int i = k - NLA_NS < 0 ? 0 : k - NLA_NS; i < k; i++)
       mbar_wait_bounded(&full[i % NLA_NS], uint32_t(i / NLA_NS) & 1u, 2000000000ull);
-    bulk_wait0();
     return;
   }
 
-  const int tid = threadIdx.x;
+  const int TS = 1 << ts, G = NLA_NT >> ts;
+  const int t = threadIdx.x & (TS - 1), g = threadIdx.x >> ts;
   T pd[J][4];
-  int pprev = -1;
-  int i = 0;
+  int pprev = -1, i = 0;
   for (long long b = blockIdx.x; b < nbatch; b += gridDim.x, i++) {
     const int st = i % NLA_NS;
-    const bool ok = wait_bar(&full[st], uint32_t(i / NLA_NS) & 1u);
-    if (nla_sync_or(!ok || *abort_flag)) break;
+    if (!wait_bar(&full[st], uint32_t(i / NLA_NS) & 1u)) break;
     const int nb = int(min((long long)KB, nrec - b * KB));
-    const int4 *rc = recs + st * NLA_KMAX;
-    T *rw = rows + size_t(st) * KB * S;
-    // the batch's first-hit coefficients, requested together
-    for (int t = tid; t < nb * 4; t += NLA_NT) hcs[t] = hcoef[(long long)rc[t >> 2].y * 4 + (t & 3)];
-    nla_sync();
-    for (int q = 0; q < nb; q++) {
-      const int4 rec = rc[q];
+    for (int q = g; q < nb; q += G) {
+      const int4 rec = recs[st * KB + q];
+      const long long pt = rec.x;
       const int h0 = rec.y, nh = rec.z, p0 = rec.w;
       if (p0 != pprev) {
 #pragma unroll
         for (int j = 0; j < J; j++) {
-          const int s = tid + j * NLA_NT;
+          const int s = t + j * TS;
           if (s < S) {
 #pragma unroll
-            for (int l = 0; l < 4; l++) pd[j][l] = projD[((long long)p0 * 4 + l) * S + s];
+            for (int l = 0; l < 4; l++) pd[j][l] = a.projD[((long long)p0 * 4 + l) * S + s];
           }
         }
         pprev = p0;
       }
       T hc[4];
 #pragma unroll
-      for (int l = 0; l < 4; l++) hc[l] = hcs[q * 4 + l];
+      for (int l = 0; l < 4; l++) hc[l] = coefs[(st * KB + q) * 4 + l];
+      T *o = a.out + pt * S;
+      T *rw = reinterpret_cast<T *>(rows + (size_t(st) * KB + q) * slot + (reinterpret_cast<uintptr_t>(o) & 15));
 #pragma unroll
       for (int j = 0; j < J; j++) {
-        const int s = tid + j * NLA_NT;
-        if (s >= S) continue;
-        T accv = mk<T>(R(0), R(0));
-#pragma unroll
-        for (int l = 0; l < 4; l++) accv = cmac(accv, hc[l], pd[j][l]);
-        for (int k = 1; k < nh; k++) {
-          const int h = h0 + k;
-          const int p = hitp[h];
-#pragma unroll
-          for (int l = 0; l < 4; l++)
-            accv = cadd(accv, cmul(hcoef[(long long)h * 4 + l], projD[((long long)p * 4 + l) * S + s]));
-        }
-        T *o = rw + (size_t)q * S + s;
-        *o = cadd(*o, scaled ? cmul(scale, accv) : accv);
+        const int s = t + j * TS;
+        if (s < S) (BS ? rw : o)[s] = nl_value<R, VM>(a, pt, s, h0, nh, rw[s], hc, pd[j]);
       }
     }
     fence_proxy_async();
-    mbar_arrive(&done[st]);  // the producer writes the rows back and refills the stage
+    mbar_arrive(&done[st]);  // the producer refills the stage
   }
 }
 
 template <typename R>
-void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, C2<R> *out, bool scaled, C2<R> scale) {
+void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, C2<R> *out, bool scaled, C2<R> scale,
+                     const R *V, int nspin, int spin, R vshift) {
   const Projectors &P = h.proj;
   if (P.nhitpts == 0) return;
-  const C2<R> *hc;
-  if constexpr (sizeof(R) == 8) hc = P.d_hcoef;
-  else hc = P.d_hcoef32;
-  // bulk form: rows of 16-byte multiples (and 16-byte aligned starts), up to 4 states per compute thread
-  const size_t row_bytes = size_t(S) * sizeof(C2<R>);
-  if (ctx.nl_bulk >= 0 && row_bytes % 16 == 0 && S <= 4 * NLA_NT && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
-    // 8 points per batch (measured at 96^3 x 256: 211 us FP32 / 318 us FP64, against 229 / 357 with
-    // 16 / 4 points and 466 / 562 with 32 / 16), fewer when a stage would pass 48 KB
-    int KB = int(49152 / row_bytes);
-    KB = KB < 1 ? 1 : (KB > 8 ? 8 : KB);
+  NlApply<R> a;
+  if constexpr (sizeof(R) == 8) a.hcoef = P.d_hcoef;
+  else a.hcoef = P.d_hcoef32;
+  a.hrec = P.d_hrec;
+  a.hitp = P.d_hitp;
+  a.projD = projD;
+  a.out = out;
+  a.S = S;
+  a.scaled = scaled;
+  a.scale = scale;
+  a.V = V;
+  a.nspin = nspin;
+  a.spin = spin;
+  a.vshift = vshift;
+  // bulk form: up to 4 states per compute thread; rows of 16-byte multiples, or sets whose last row's copy
+  // ends inside them
+  const size_t row_bytes = size_t(S) * sizeof(C2<R>), slot = (row_bytes + 15) & ~size_t(15);
+  const bool whole = row_bytes % 16 == 0 || (size_t(h.basis->npoints) * S) % 2 == 0;
+  // (rows below 256 bytes leave the bulk form to option 1: 24^3 x 9 single 3.4 us against 2.9, 64^3 x 8 FP64 16 against 13)
+  if (ctx.nl_bulk >= 0 && (ctx.nl_bulk > 0 || row_bytes >= 256) && whole && S <= 4 * NLA_NT && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
+    // 8 points per batch, 16 for rows of at most 1 KB when there are many (measured at 120^3 x 64 FP64, 440 k
+    // points: 186 us with 8, 162 with 16, 164 with 32; 40^3 x 50 single, 14 k points: 6.5, -, 8.5)
+    int KB = slot <= 1024 && P.nhitpts / 16 >= 32LL * ctx.device_sms ? 16 : 8;
+    if (KB > int(49152 / slot)) KB = int(49152 / slot);
+    if (KB < 1) KB = 1;
     if (ctx.nl_apply_points > 0) KB = ctx.nl_apply_points;
-    const size_t smem = size_t(NLA_NS) * KB * row_bytes + NLA_KMAX * 4 * sizeof(C2<R>) + NLA_NS * NLA_KMAX * sizeof(int4) +
-                        2 * NLA_NS * sizeof(uint64_t) + 16;
+    const size_t smem = size_t(NLA_NS) * KB * (slot + 4 * sizeof(C2<R>) + sizeof(int4)) + 2 * NLA_NS * sizeof(uint64_t) + 16;
     if (smem <= size_t(ctx.max_smem_optin)) {
-      auto kern = S <= 2 * NLA_NT ? nl_apply_bulk_kernel<R, 2> : nl_apply_bulk_kernel<R, 4>;
+      const bool bs = row_bytes % 16 == 0 && row_bytes >= 1024;
+      const bool vm = V != nullptr;
+      using Kern = void (*)(NlApply<R>, long long, int, int, int *);
+      static const Kern kerns[12] = {
+          nl_apply_bulk_kernel<R, 1, false, false>, nl_apply_bulk_kernel<R, 2, false, false>, nl_apply_bulk_kernel<R, 4, false, false>,
+          nl_apply_bulk_kernel<R, 1, true, false>,  nl_apply_bulk_kernel<R, 2, true, false>,  nl_apply_bulk_kernel<R, 4, true, false>,
+          nl_apply_bulk_kernel<R, 1, false, true>,  nl_apply_bulk_kernel<R, 2, false, true>,  nl_apply_bulk_kernel<R, 4, false, true>,
+          nl_apply_bulk_kernel<R, 1, true, true>,   nl_apply_bulk_kernel<R, 2, true, true>,   nl_apply_bulk_kernel<R, 4, true, true>};
+      // states per thread 1, 2 or 4; rows copied out or stored; with or without the local potential
+      const int ki = (S <= NLA_NT ? 0 : (S <= 2 * NLA_NT ? 1 : 2)) + (bs ? 3 : 0) + (vm ? 6 : 0);
+      const Kern kern = kerns[ki];
+      int ts = 7;  // threads per row: a power of two from 8 to 128
+      while (ts > 3 && (1 << (ts - 1)) >= S) ts--;
       ensure_smem_attr(reinterpret_cast<const void *>(kern), smem);
       // CTAs per SM for this kernel and shared-memory size, computed once under a lock
       static std::mutex mtx;
-      static const void *occ_kern[2] = {nullptr, nullptr};
-      static size_t occ_smem[2] = {0, 0};
-      static int occ_per_sm[2] = {1, 1};
-      const int slot = S <= 2 * NLA_NT ? 0 : 1;
+      static size_t occ_smem[12] = {};
+      static int occ_per_sm[12] = {};
       int per_sm;
       {
         std::lock_guard<std::mutex> lock(mtx);
-        if (occ_kern[slot] != reinterpret_cast<const void *>(kern) || occ_smem[slot] != smem) {
-          INQB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_per_sm[slot], kern, NLA_NT + 32, smem));
-          occ_kern[slot] = reinterpret_cast<const void *>(kern);
-          occ_smem[slot] = smem;
+        if (occ_smem[ki] != smem) {
+          INQB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_per_sm[ki], kern, NLA_NT + 32, smem));
+          occ_smem[ki] = smem;
         }
-        per_sm = occ_per_sm[slot];
+        per_sm = occ_per_sm[ki];
       }
       const long long nbatch = (P.nhitpts + KB - 1) / KB;
       long long grid = (long long)(per_sm < 1 ? 1 : per_sm) * ctx.num_sms;
       if (grid > nbatch) grid = nbatch;
-      kern<<<unsigned(grid), NLA_NT + 32, smem, ctx.stream>>>(P.nhitpts, KB, S, P.d_hrec, P.d_hitp, hc, projD, out,
-                                                             scaled, scale, ctx.d_err);
+      kern<<<unsigned(grid), NLA_NT + 32, smem, ctx.stream>>>(a, P.nhitpts, KB, ts, ctx.d_err);
       LAUNCHED(ctx);
       return;
     }
   }
-  const int chunk = 32 * int(16 / sizeof(R));
+  int sl = 5;
+  while (sl > 2 && (1 << (sl - 1)) >= S) sl--;
+  constexpr int U = 16 / int(sizeof(R));  // states per lane: 4 single, 2 double; 1 when a warp holds them all
+  const int chunk = S <= 32 ? 1 << sl : U << sl;
   const int nchunks = (S + chunk - 1) / chunk;
   const long long nitems = P.nhitpts * nchunks;
-  long long blocks = (nitems + 3) / 4;
+  long long blocks = ((nitems << sl) + 127) / 128;
   if (blocks > 148LL * 48) blocks = 148LL * 48;
-  nl_apply_kernel<R><<<unsigned(blocks), 128, 0, ctx.stream>>>(nitems, nchunks, S, P.d_hrec, P.d_hitp, hc, projD, out,
-                                                               scaled, scale);
+  using Kern = void (*)(NlApply<R>, long long, int, int);
+  const Kern kern = S <= 32 ? (V ? Kern(nl_apply_kernel<R, 1, true>) : Kern(nl_apply_kernel<R, 1, false>))
+                            : (V ? Kern(nl_apply_kernel<R, U, true>) : Kern(nl_apply_kernel<R, U, false>));
+  kern<<<unsigned(blocks), 128, 0, ctx.stream>>>(a, nitems, nchunks, sl);
   LAUNCHED(ctx);
 }
 
@@ -1909,7 +1986,8 @@ void launch_taylor_combine(Ctx &ctx, const C2<R> *x, const C2<R> *const *u, int 
   template void launch_nl_project<R>(Ctx &, const Basis &, const Hamiltonian &, const C2<R> *, int, C2<R> *,       \
                                      C2<R> *);                                                                    \
   template void launch_nl_scatter<R>(Ctx &, const Basis &, const Hamiltonian &, const C2<R> *, int, C2<R> *);     \
-  template void launch_nl_apply<R>(Ctx &, const Hamiltonian &, const C2<R> *, int, C2<R> *, bool, C2<R>);        \
+  template void launch_nl_apply<R>(Ctx &, const Hamiltonian &, const C2<R> *, int, C2<R> *, bool, C2<R>, const R *, \
+                                   int, int, R);                                                                  \
   template void launch_taylor_combine<R>(Ctx &, const C2<R> *, const C2<R> *const *, int, const double2 *,         \
                                          const double2 *, C2<R> *, C2<R> *, long long);                           \
   template void launch_fill<R>(Ctx &, C2<R> *, long long, double, double);                                         \
