@@ -794,25 +794,33 @@ template <typename R> void load_states(Orbitals &phi, const std::string &dir) {
 
 // ============================================================================ C ABI
 
-// operations::orthogonalize (orthogonalize.hpp:25-31)
+// operations::orthogonalize (orthogonalize.hpp:25-31), all on the device; the host only learns whether the
+// overlap was positive definite (if not, the set is left as it is)
 void orthogonalize_dev(Orbitals &phi) {
   Ctx &ctx = *phi.ctx;
   const int S = phi.nst;
   double2 *d = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * S * S));
+  double2 *X = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * S * S));
+  int *bad_dev = static_cast<int *>(dev_alloc(ctx, sizeof(int)));
   overlap_dev(phi, phi, d);
-  auto Sh = download<std::complex<double>>(ctx, d, size_t(S) * S);
-  std::vector<std::complex<double>> X(size_t(S) * S);
-  cholesky_inverse(S, Sh.data(), X.data());
-  INQB_CUDA(cudaMemcpyAsync(d, X.data(), sizeof(double2) * S * S, cudaMemcpyHostToDevice, ctx.stream));
-  rotate_dev(phi, d);
+  launch_cholesky_inverse(ctx, S, d, X, bad_dev);
+  if (!ctx.fp64_mma) {  // SIMT products: the full rotation, once the host knows that there is a factor
+    if (download<int>(ctx, bad_dev, 1)[0] == 0) rotate_dev(phi, X);
+  } else if (phi.precision == INQB_F64)
+    launch_rotate_upper<double>(ctx, static_cast<double2 *>(phi.data), S, phi.basis->npoints, X, bad_dev);
+  else
+    launch_rotate_upper<float>(ctx, static_cast<float2 *>(phi.data), S, phi.basis->npoints, X, bad_dev);
+  const auto bad = download<int>(ctx, bad_dev, 1);
+  dev_free(ctx, bad_dev);
+  dev_free(ctx, X);
   dev_free(ctx, d);
-  INQB_CUDA(cudaStreamSynchronize(ctx.stream));
+  INQB_REQUIRE(bad[0] == 0, INQB_ERR_NUMERIC, "overlap matrix is not positive definite (orthogonalize)");
 }
 
 // eigensolvers::steepest_descent (steepest_descent.hpp:23-86) with the Teter-Payne-Allan preconditioner
 // (preconditioner.hpp:24-46) on a Fourier-space set: five line-minimisation steps per state along the
-// preconditioned residual, then orthogonalize.  The per-state overlaps are FP64 reductions; the step
-// lengths are formed on the host.
+// preconditioned residual, then orthogonalize.  The per-state overlaps are FP64 reductions, and the step
+// lengths are formed on the device: a step is H on the residual and five passes over the sets.
 template <typename R> void steepest_descent_t(Hamiltonian &h, Orbitals &phi) {
   Ctx &ctx = *h.ctx;
   const Basis &b = *h.basis;
@@ -820,54 +828,18 @@ template <typename R> void steepest_descent_t(Hamiltonian &h, Orbitals &phi) {
   const long long np = b.npoints;
   using T = C2<R>;
   constexpr int num_steps = 5;
-  TempSet hphi(phi), res(phi), hres(phi), lap(phi);
+  TempSet hphi(phi), res(phi), hres(phi);
   auto D = [](Orbitals &o) { return static_cast<T *>(o.data); };
-  auto CD = [](const Orbitals &o) { return static_cast<const T *>(o.data); };
-  double2 *dov = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * S));
-  double2 *dcoef = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * S));
-  double *dkin = static_cast<double *>(dev_alloc(ctx, sizeof(double) * S));
-  auto ovd = [&](const Orbitals &x, const Orbitals &y) {
-    ovdiag_dev(x, y, dov);
-    return download<std::complex<double>>(ctx, dov, size_t(S));
-  };
+  const double dv = set_volume_element(phi);
+  void *work = dev_alloc(ctx, launch_sd_work_bytes(S));
   apply_any(h, phi, hphi.o);
-  std::vector<double2> coef(S);
-  std::vector<double> kin(S);
-  const double zero[3] = {0.0, 0.0, 0.0};
+  launch_sd_rayleigh<R>(ctx, D(phi), D(hphi.o), S, np, dv, work);
   for (int istep = 0; istep < num_steps; istep++) {
-    copy_set(hphi.o, res.o);
-    const auto ev = ovd(res.o, phi);
-    const auto nrm = ovd(phi, phi);
-    for (int s = 0; s < S; s++) {
-      const std::complex<double> e = ev[s] / nrm[s].real();
-      coef[s] = make_double2(e.real(), e.imag());
-    }
-    INQB_CUDA(cudaMemcpyAsync(dcoef, coef.data(), sizeof(double2) * S, cudaMemcpyHostToDevice, ctx.stream));
-    launch_shift_cvec<R>(ctx, D(res.o), CD(phi), S, np, dcoef, -1.0);
-    // preconditioner: kinetic energy per state, then K(0.5 |G|^2 / T_s)
-    launch_laplacian<R>(ctx, b, CD(res.o), D(lap.o), S, -0.5, zero);
-    const auto tv = ovd(lap.o, res.o);
-    const auto tn = ovd(res.o, res.o);
-    for (int s = 0; s < S; s++) kin[s] = (tv[s] / tn[s]).real();
-    INQB_CUDA(cudaMemcpyAsync(dkin, kin.data(), sizeof(double) * S, cudaMemcpyHostToDevice, ctx.stream));
-    launch_tpa_precondition<R>(ctx, b, D(res.o), S, dkin);
+    launch_sd_residual<R>(ctx, b, D(phi), D(hphi.o), D(res.o), S, dv, work);
     apply_any(h, res.o, hres.o);
-    const auto m0 = ovd(res.o, res.o), m1 = ovd(phi, res.o), m2 = ovd(res.o, hres.o), m3 = ovd(phi, hres.o);
-    for (int s = 0; s < S; s++) {
-      const double ca = (m0[s] * m3[s] - m2[s] * m1[s]).real();
-      const double cb = (nrm[s] * m2[s] - ev[s] * m0[s]).real();
-      const double cc = (ev[s] * m1[s] - m3[s] * nrm[s]).real();
-      const double den = cb + std::sqrt(cb * cb - 4.0 * ca * cc);
-      coef[s] = make_double2(std::fabs(den) < 1e-15 ? 0.0 : 2.0 * cc / den, 0.0);
-    }
-    INQB_CUDA(cudaMemcpyAsync(dcoef, coef.data(), sizeof(double2) * S, cudaMemcpyHostToDevice, ctx.stream));
-    launch_shift_cvec<R>(ctx, D(phi), CD(res.o), S, np, dcoef, 1.0);
-    if (istep != num_steps - 1) launch_shift_cvec<R>(ctx, D(hphi.o), CD(hres.o), S, np, dcoef, 1.0);
+    launch_sd_update<R>(ctx, D(phi), D(hphi.o), D(res.o), D(hres.o), S, np, dv, work, istep == num_steps - 1);
   }
-  INQB_CUDA(cudaStreamSynchronize(ctx.stream));  // the host factors above go out of scope
-  dev_free(ctx, dov);
-  dev_free(ctx, dcoef);
-  dev_free(ctx, dkin);
+  dev_free(ctx, work);
 }
 
 extern "C" {
@@ -2012,11 +1984,33 @@ int inqb_subspace_diagonalization(const inqb_hamiltonian *hc, inqb_orbitals *phi
       apply_any(*h, *phi, hp.o);
       overlap_dev(*phi, hp.o, d);
     }
-    auto Hs = download<std::complex<double>>(ctx, d, size_t(S) * S);
-    std::vector<std::complex<double>> V(size_t(S) * S);
-    hermitian_eigen(S, Hs.data(), eigenvalues, V.data());
-    // phi_k <- sum_j V[j][k] phi_j (operations::rotate with the eigenvectors, rotate.hpp:27-62)
-    INQB_CUDA(cudaMemcpyAsync(d, V.data(), sizeof(double2) * S * S, cudaMemcpyHostToDevice, ctx.stream));
+    // eigenvalues in ascending order; phi_k <- sum_j V[j][k] phi_j (operations::rotate, rotate.hpp:27-62)
+    if (S <= 13) {
+      // few states: the host's rotations take less time than the device's chain of waves (12 states 0.4 against
+      // 0.5 ms, 16 states 1.1 against 0.65)
+      const auto Hs = download<std::complex<double>>(ctx, d, size_t(S) * S);
+      std::vector<std::complex<double>> V(size_t(S) * S);
+      hermitian_eigen(S, Hs.data(), eigenvalues, V.data());
+      INQB_CUDA(cudaMemcpyAsync(d, V.data(), sizeof(double2) * S * S, cudaMemcpyHostToDevice, ctx.stream));
+      rotate_dev(*phi, d);
+      dev_free(ctx, d);
+      INQB_CUDA(cudaStreamSynchronize(ctx.stream));
+      return;
+    }
+    double2 *V = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * S * S));
+    double *w_dev = static_cast<double *>(dev_alloc(ctx, sizeof(double) * S));
+    int *order_dev = static_cast<int *>(dev_alloc(ctx, sizeof(int) * S));
+    launch_jacobi(ctx, S, d, V, w_dev);
+    const auto w = download<double>(ctx, w_dev, size_t(S));
+    std::vector<int> order(S);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return w[x] < w[y]; });
+    for (int k = 0; k < S; k++) eigenvalues[k] = w[order[k]];
+    INQB_CUDA(cudaMemcpyAsync(order_dev, order.data(), sizeof(int) * S, cudaMemcpyHostToDevice, ctx.stream));
+    launch_permute_columns(ctx, V, order_dev, S, d);
+    dev_free(ctx, order_dev);
+    dev_free(ctx, w_dev);
+    dev_free(ctx, V);
     rotate_dev(*phi, d);
     dev_free(ctx, d);
     INQB_CUDA(cudaStreamSynchronize(ctx.stream));

@@ -259,6 +259,12 @@ void launch_eigen_sums(Ctx &ctx, const C2<R> *a, const C2<R> *b, int S, long lon
                        double2 *ne_dev /*[S]*/, double2 *res_dev /*[S] or null*/);
 template <typename R>
 void launch_rotate(Ctx &ctx, C2<R> *phi, int S, long long npoints, const double2 *Rdev);
+template <typename R>
+void launch_rotate_upper(Ctx &ctx, C2<R> *phi, int S, long long npoints, const double2 *X, const int *skip_dev);
+// dense Hermitian matrices on the device (dense.cu)
+void launch_cholesky_inverse(Ctx &ctx, int n, double2 *S, double2 *X, int *bad_dev);
+void launch_jacobi(Ctx &ctx, int n, double2 *A, double2 *V, double *w_dev);
+void launch_permute_columns(Ctx &ctx, const double2 *V, const int *order_dev, int n, double2 *out);
 void launch_wait_timeout(Ctx &ctx, long long limit_ns);
 // dipole.hpp:24-60 of a device density [npoints]: out3_dev = dV sum_r n(r) r
 void launch_dipole(Ctx &ctx, const Basis &b, const double *dens, double *out3_dev);
@@ -272,7 +278,17 @@ template <typename R> void launch_kick(Ctx &ctx, const Basis &b, C2<R> *phi, int
 template <typename R>
 void launch_shift_cvec(Ctx &ctx, C2<R> *y, const C2<R> *x, int S, long long npoints, const double2 *coef_dev,
                        double scale);
-template <typename R> void launch_tpa_precondition(Ctx &ctx, const Basis &b, C2<R> *x, int S, const double *kin_dev);
+// steepest-descent passes (reduce.cu) over Fourier-space sets; `work` holds launch_sd_work_bytes(S) bytes and
+// carries the coefficients from one to the next: Rayleigh sums; preconditioned residual; line minimisation
+size_t launch_sd_work_bytes(int S);
+template <typename R>
+void launch_sd_rayleigh(Ctx &ctx, const C2<R> *phi, const C2<R> *hphi, int S, long long npoints, double dv, void *work);
+template <typename R>
+void launch_sd_residual(Ctx &ctx, const Basis &b, const C2<R> *phi, const C2<R> *hphi, C2<R> *res, int S, double dv,
+                        void *work);
+template <typename R>
+void launch_sd_update(Ctx &ctx, C2<R> *phi, C2<R> *hphi, const C2<R> *res, const C2<R> *hres, int S, long long npoints,
+                      double dv, void *work, bool last);
 // states [s0, s0 + ns) of a [np][S] set to / from contiguous complex128 rows [ns][np]
 template <typename R>
 void launch_extract_states(Ctx &ctx, const C2<R> *in, int S, long long np, int s0, int ns, double2 *out);

@@ -904,140 +904,6 @@ void launch_laplacian(Ctx &ctx, const Basis &b, const C2<R> *in, C2<R> *out, int
   LAUNCHED(ctx);
 }
 
-// ------------------------------------------------------------------ per-state reductions
-// Stage 1: block b handles a contiguous point range; thread t owns state s = t (blockDim >= S handled by loop)
-// and accumulates over its points in a fixed order: U running sums over the points p = 0 .. U-1 mod U of the
-// range (U independent loads of each operand in flight per thread; U = 8 for single precision, whose 8-byte
-// elements need twice the loads in flight to cover the same bytes), added pairwise at the end.  Stage 2
-// sums the block partials in order.  592 blocks of 256 threads are resident at once (4 per SM).
-constexpr int RED_BLOCKS = 592;
-
-// MODE 0: conj(a) b; 1: conj(a) lapl a; 2: |b - e_s a|^2 (the residual norm of energy.hpp:86-89 without
-// forming the residual); 3: (|a|^2, Re conj(a) b), the two sums of one eigenvalue in one pass
-template <typename R, int MODE>
-__device__ __forceinline__ double2 state_term(const C2<R> *__restrict__ a, const C2<R> *__restrict__ b, int S,
-                                              long long p, int s, const Metric &m, double factor, const Vec3 &gc,
-                                              double k2, double es) {
-  const C2<R> x = a[p * S + s];
-  if (MODE == 0) {
-    const C2<R> y = b[p * S + s];
-    return make_double2(double(x.x) * double(y.x) + double(x.y) * double(y.y),
-                        double(x.x) * double(y.y) - double(x.y) * double(y.x));
-  } else if (MODE == 1) {
-    const double f = lapl_at(m, p, factor, gc.v, k2);
-    return make_double2(f * (double(x.x) * double(x.x) + double(x.y) * double(x.y)), 0.0);
-  } else if (MODE == 2) {
-    const C2<R> y = b[p * S + s];
-    const double rx = double(y.x) - es * double(x.x), ry = double(y.y) - es * double(x.y);
-    return make_double2(rx * rx + ry * ry, 0.0);
-  } else {
-    const C2<R> y = b[p * S + s];
-    return make_double2(double(x.x) * double(x.x) + double(x.y) * double(x.y),
-                        double(x.x) * double(y.x) + double(x.y) * double(y.y));
-  }
-}
-
-template <typename R, int MODE>
-__global__ void state_reduce_kernel(const C2<R> *__restrict__ a, const C2<R> *__restrict__ b, int S, long long npoints,
-                                    Metric m, double factor, Vec3 gc, double k2, const double2 *__restrict__ ne,
-                                    double2 *partial) {
-  const long long chunk = (npoints + gridDim.x - 1) / gridDim.x;
-  const long long p0 = blockIdx.x * chunk;
-  const long long p1 = min(npoints, p0 + chunk);
-  constexpr int U = sizeof(R) == 4 ? 8 : 4;
-  for (int s = threadIdx.x; s < S; s += blockDim.x) {
-    // MODE 2: the eigenvalue Re<a|b>/<a|a> from the MODE 3 sums (the same division the host does)
-    const double es = MODE == 2 ? ne[s].y / ne[s].x : 0.0;
-    double2 acc[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) acc[u] = make_double2(0.0, 0.0);
-    long long p = p0;
-    for (; p + U - 1 < p1; p += U) {
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const double2 t = state_term<R, MODE>(a, b, S, p + u, s, m, factor, gc, k2, es);
-        acc[u].x += t.x;
-        acc[u].y += t.y;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U - 1; u++)
-      if (p + u < p1) {
-        const double2 t = state_term<R, MODE>(a, b, S, p + u, s, m, factor, gc, k2, es);
-        acc[u].x += t.x;
-        acc[u].y += t.y;
-      }
-#pragma unroll
-    for (int w = U / 2; w >= 1; w /= 2)
-#pragma unroll
-      for (int u = 0; u < w; u++) {
-        acc[u].x += acc[u + w].x;
-        acc[u].y += acc[u + w].y;
-      }
-    partial[(long long)blockIdx.x * S + s] = acc[0];
-  }
-}
-
-__global__ void sum_partials_kernel(const double2 *partial, int nblk, int S, double scale, double2 *out) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
-    double re = 0.0, im = 0.0;
-    for (int k = 0; k < nblk; k++) {
-      re += partial[(long long)k * S + s].x;
-      im += partial[(long long)k * S + s].y;
-    }
-    out[s] = make_double2(scale * re, scale * im);
-  }
-}
-
-template <typename R>
-void launch_overlap_diag(Ctx &ctx, const C2<R> *a, const C2<R> *b, int S, long long npoints, double dv, double2 *out) {
-  double2 *partial = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * RED_BLOCKS * S));
-  Metric m{};
-  Vec3 g{{0, 0, 0}};
-  state_reduce_kernel<R, 0><<<RED_BLOCKS, 256, 0, ctx.stream>>>(a, b, S, npoints, m, 0.0, g, 0.0, nullptr, partial);
-  LAUNCHED(ctx);
-  sum_partials_kernel<<<(S + 255) / 256, 256, 0, ctx.stream>>>(partial, RED_BLOCKS, S, dv, out);
-  LAUNCHED(ctx);
-  dev_free(ctx, partial);
-}
-
-// Eigenvalues and residual norms of energy.hpp:80-89 in two passes over a and b = H a:
-// ne[s] = dv (<a|a>, Re<a|b>); when res is given, res[s].x = dv sum_p |b - e_s a|^2 with e_s = ne[s].y / ne[s].x
-template <typename R>
-void launch_eigen_sums(Ctx &ctx, const C2<R> *a, const C2<R> *b, int S, long long npoints, double dv, double2 *ne,
-                       double2 *res) {
-  double2 *partial = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * RED_BLOCKS * S));
-  Metric m{};
-  Vec3 g{{0, 0, 0}};
-  state_reduce_kernel<R, 3><<<RED_BLOCKS, 256, 0, ctx.stream>>>(a, b, S, npoints, m, 0.0, g, 0.0, nullptr, partial);
-  LAUNCHED(ctx);
-  sum_partials_kernel<<<(S + 255) / 256, 256, 0, ctx.stream>>>(partial, RED_BLOCKS, S, dv, ne);
-  LAUNCHED(ctx);
-  if (res) {
-    state_reduce_kernel<R, 2><<<RED_BLOCKS, 256, 0, ctx.stream>>>(a, b, S, npoints, m, 0.0, g, 0.0, ne, partial);
-    LAUNCHED(ctx);
-    sum_partials_kernel<<<(S + 255) / 256, 256, 0, ctx.stream>>>(partial, RED_BLOCKS, S, dv, res);
-    LAUNCHED(ctx);
-  }
-  dev_free(ctx, partial);
-}
-
-template <typename R>
-void launch_kinetic_ev(Ctx &ctx, const Basis &b, const C2<R> *fphi, int S, double factor, const double gc[3], double k2,
-                       double *out_dev) {
-  double2 *partial = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * (RED_BLOCKS * S + S)));
-  Vec3 g{{gc[0], gc[1], gc[2]}};
-  state_reduce_kernel<R, 1><<<RED_BLOCKS, 256, 0, ctx.stream>>>(fphi, fphi, S, b.npoints, metric_of(b), factor, g, k2, nullptr,
-                                                                partial);
-  LAUNCHED(ctx);
-  double2 *sums = partial + RED_BLOCKS * S;
-  sum_partials_kernel<<<(S + 255) / 256, 256, 0, ctx.stream>>>(partial, RED_BLOCKS, S, 1.0, sums);
-  LAUNCHED(ctx);
-  INQB_CUDA(cudaMemcpy2DAsync(out_dev, sizeof(double), sums, sizeof(double2), sizeof(double), S,
-                              cudaMemcpyDeviceToDevice, ctx.stream));
-  dev_free(ctx, partial);
-}
-
 // ------------------------------------------------------------------ overlap (complex GEMM, K = npoints)
 // S[i][j] = dv * sum_p conj(a[p][i]) b[p][j].  64x64 output tile per CTA, split-K over point chunks,
 // 256 threads with a 4x4 register tile each, two CTAs per SM (128 registers: 24.5 ms against 31.6 ms with
@@ -1277,11 +1143,17 @@ __global__ void __launch_bounds__(128) overlap64_mma_kernel(const double2 *__res
       }
 }
 
-__global__ void sum_tiles_kernel(const double2 *partial, int nz, long long n, int S, int sym, double scale,
-                                 double2 *out) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+// out = scale * the chunks' tiles, summed in eight slices of the chunks (each in order, then the slices in
+// order); block = 32 elements x 8 slices (one thread per element adding up to 256 chunks took 29 us)
+__global__ void __launch_bounds__(256) sum_tiles_kernel(const double2 *partial, int nz, long long n, int S, int sym,
+                                                        double scale, double2 *out) {
+  __shared__ double2 red[8][32];
+  const int c = threadIdx.x % 32, sl = threadIdx.x / 32;
+  const long long e = blockIdx.x * 32LL + c;
+  bool mirror = false;
+  double re = 0.0, im = 0.0;
+  if (e < n) {
     long long src = e;
-    bool mirror = false;
     if (sym) {
       const int i = int(e / S), j = int(e % S);
       if (i / 64 > j / 64) {
@@ -1289,10 +1161,20 @@ __global__ void sum_tiles_kernel(const double2 *partial, int nz, long long n, in
         mirror = true;
       }
     }
-    double re = 0.0, im = 0.0;
-    for (int z = 0; z < nz; z++) {
-      re += partial[z * n + src].x;
-      im += partial[z * n + src].y;
+    const int per = (nz + 7) / 8, z1 = min(nz, (sl + 1) * per);
+#pragma unroll 8
+    for (int z = sl * per; z < z1; z++) {
+      const double2 v = partial[z * n + src];
+      re += v.x;
+      im += v.y;
+    }
+  }
+  red[sl][c] = make_double2(re, im);
+  __syncthreads();
+  if (sl == 0 && e < n) {
+    for (int q = 1; q < 8; q++) {
+      re += red[q][c].x;
+      im += red[q][c].y;
     }
     out[e] = make_double2(scale * re, mirror ? -scale * im : scale * im);
   }
@@ -1329,7 +1211,7 @@ void launch_overlap(Ctx &ctx, const C2<R> *a, int Sa, const C2<R> *b, int Sb, lo
   }
   LAUNCHED(ctx);
   const long long n = (long long)Sa * Sb;
-  sum_tiles_kernel<<<grid_for(n, 256), 256, 0, ctx.stream>>>(partial, nz, n, Sb, sym, dv, out);
+  sum_tiles_kernel<<<unsigned((n + 31) / 32), 256, 0, ctx.stream>>>(partial, nz, n, Sb, sym, dv, out);
   LAUNCHED(ctx);
   dev_free(ctx, partial);
 }
@@ -1484,30 +1366,48 @@ __global__ void __launch_bounds__(256, 2) rotate_tiled_kernel(const C2<R> *__res
 // re.re - im.im into the real part, re.im + im.re into the imaginary): 64 points x 64 output states per
 // CTA of 128 threads, each warp a 32 x 32 block of 8 x 8 fragments; operand tiles double-buffered by
 // cp.async, rows padded (20 elements of in, 66 of R) so that the fragment loads hit distinct banks.
-template <typename R>
-__global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *__restrict__ in, int Sin, C2<R> *__restrict__ out,
+// UPPER: Rm is upper triangular, in == out and Sin == Sout.  A CTA takes all output tiles of its 64 points,
+// from the last to the first: tile j needs the input states up to its own last one only, so it skips the
+// zeros below (5/8 of the products at 256 states), and overwrites states that no later tile reads, so no
+// scratch block and copy back are needed.  *skip != 0 leaves the set as it is.
+template <typename R, bool UPPER>
+__global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *in, int Sin, C2<R> *out,
                                                          int Sout, long long npoints, const double2 *__restrict__ Rm,
-                                                         double2 alpha, double2 beta, int scaled, int use_beta) {
+                                                         double2 alpha, double2 beta, int scaled, int use_beta,
+                                                         const int *skip) {
   using T = C2<R>;
+  if (UPPER && *skip) return;
   constexpr int TP = 64, TJ = 64, KT = 16, LDA = 20, LDB = TJ + 2;
   constexpr int EPC = 16 / int(sizeof(T));  // elements of in per 16-byte copy
   extern __shared__ __align__(16) unsigned char rsm[];
   T *Abuf = reinterpret_cast<T *>(rsm);                                   // [2][TP][LDA]
   double2 *Bbuf = reinterpret_cast<double2 *>(Abuf + 2 * TP * LDA);       // [2][KT][LDB]
   const int njt = (Sout + TJ - 1) / TJ;
-  const int j0 = int(blockIdx.x % njt) * TJ;
-  const long long p0 = (long long)(blockIdx.x / njt) * TP;
+  const long long p0 = (long long)(UPPER ? blockIdx.x : blockIdx.x / njt) * TP;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
   const int fk = lane & 3, fs = lane >> 2;
+  const bool whole = (size_t(Sin) * sizeof(T)) % 16 == 0;  // rows of 16-byte multiples; else 8-byte copies
+  for (int jt = UPPER ? njt - 1 : int(blockIdx.x % njt), last = UPPER ? 0 : jt; jt >= last; jt--) {
+  const int j0 = jt * TJ;
+  const int kend = UPPER && j0 + TJ < Sin ? j0 + TJ : Sin;
   auto issue = [&](int buf, int k0) {
     T *As = Abuf + buf * TP * LDA;
     double2 *Bs = Bbuf + buf * KT * LDB;
-    for (int e = threadIdx.x; e < TP * KT / EPC; e += 128) {
-      const int r = e / (KT / EPC), kk = (e % (KT / EPC)) * EPC;
-      const long long p = p0 + r;
-      const bool v = p < npoints && k0 + kk < Sin;
-      ptx::cp_async16(As + r * LDA + kk, v ? in + p * Sin + k0 + kk : in, v ? 16u : 0u);
+    if (sizeof(T) == 16 || whole) {
+      for (int e = threadIdx.x; e < TP * KT / EPC; e += 128) {
+        const int r = e / (KT / EPC), kk = (e % (KT / EPC)) * EPC;
+        const long long p = p0 + r;
+        const bool v = p < npoints && k0 + kk < Sin;
+        ptx::cp_async16(As + r * LDA + kk, v ? in + p * Sin + k0 + kk : in, v ? 16u : 0u);
+      }
+    } else {
+      for (int e = threadIdx.x; e < TP * KT; e += 128) {
+        const int r = e / KT, kk = e % KT;
+        const long long p = p0 + r;
+        if (p < npoints && k0 + kk < Sin) ptx::cp_async8(As + r * LDA + kk, in + p * Sin + k0 + kk);
+        else As[r * LDA + kk] = mk<T>(R(0), R(0));
+      }
     }
     for (int e = threadIdx.x; e < KT * TJ; e += 128) {
       const int kk = e / TJ, c = e % TJ;
@@ -1523,8 +1423,8 @@ __global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *__restrict
     for (int v = 0; v < 4; v++) cre[u][v][0] = cre[u][v][1] = cim[u][v][0] = cim[u][v][1] = 0.0;
   issue(0, 0);
   int cur = 0;
-  for (int k0 = 0; k0 < Sin; k0 += KT, cur ^= 1) {
-    if (k0 + KT < Sin) {
+  for (int k0 = 0; k0 < kend; k0 += KT, cur ^= 1) {
+    if (k0 + KT < kend) {
       issue(cur ^ 1, k0 + KT);
       ptx::cp_async_wait<1>();
     } else {
@@ -1533,6 +1433,7 @@ __global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *__restrict
     __syncthreads();
     const T *As = Abuf + cur * TP * LDA;
     const double2 *Bs = Bbuf + cur * KT * LDB;
+    if (!UPPER || k0 < j0 + wn + 32) {  // the warp's 32 columns end above row k0
 #pragma unroll
     for (int ks = 0; ks < KT; ks += 4) {
       double2 af[4], bf[4];
@@ -1552,6 +1453,7 @@ __global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *__restrict
           dmma_8x8x4(cim[u][v], af[u].x, bf[v].y);
           dmma_8x8x4(cim[u][v], af[u].y, bf[v].x);
         }
+    }
     }
     __syncthreads();
   }
@@ -1575,6 +1477,7 @@ __global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *__restrict
           *o = mk<T>(R(w.x), R(w.y));
         }
       }
+  }
 }
 
 // out <- alpha (in Rm) + beta out, Rm [Sin][Sout]; in == out (Sin == Sout) rotates in place
@@ -1590,14 +1493,14 @@ void launch_rotate_to(Ctx &ctx, const C2<R> *in, int Sin, C2<R> *out, int Sout, 
     // copied back (the kernel's CTAs for one tile of points read all of its states)
     const size_t tsmem = 2 * 64 * 16 * sizeof(C2<R>) + 2 * 16 * 64 * sizeof(double2);
     const size_t msmem = 2 * 64 * 20 * sizeof(C2<R>) + 2 * 16 * 66 * sizeof(double2);
-    if (ctx.fp64_mma) ensure_smem_attr(reinterpret_cast<const void *>(rotate_mma_kernel<R>), msmem);
+    if (ctx.fp64_mma) ensure_smem_attr(reinterpret_cast<const void *>(rotate_mma_kernel<R, false>), msmem);
     else ensure_smem_attr(reinterpret_cast<const void *>(rotate_tiled_kernel<R>), tsmem);
     auto launch = [&](const C2<R> *src, C2<R> *dst, long long n) {
       const long long nblk = (long long)((Sout + 63) / 64) * ((n + 63) / 64);
       INQB_REQUIRE(nblk < (1LL << 31), INQB_ERR_UNSUPPORTED, "set too large for the rotation grid");
       if (ctx.fp64_mma)
-        rotate_mma_kernel<R><<<unsigned(nblk), 128, msmem, ctx.stream>>>(src, Sin, dst, Sout, n, Rdev, alpha, beta,
-                                                                         scaled, use_beta);
+        rotate_mma_kernel<R, false><<<unsigned(nblk), 128, msmem, ctx.stream>>>(src, Sin, dst, Sout, n, Rdev, alpha, beta,
+                                                                                scaled, use_beta, nullptr);
       else
         rotate_tiled_kernel<R><<<unsigned(nblk), 256, tsmem, ctx.stream>>>(src, Sin, dst, Sout, n, Rdev, alpha, beta,
                                                                           scaled, use_beta);
@@ -1628,34 +1531,57 @@ void launch_rotate_to(Ctx &ctx, const C2<R> *in, int Sin, C2<R> *out, int Sout, 
   LAUNCHED(ctx);
 }
 
+// phi <- phi X in place with X upper triangular, unless *skip_dev
+template <typename R>
+void launch_rotate_upper(Ctx &ctx, C2<R> *phi, int S, long long npoints, const double2 *X, const int *skip_dev) {
+  const size_t smem = 2 * 64 * 20 * sizeof(C2<R>) + 2 * 16 * 66 * sizeof(double2);
+  ensure_smem_attr(reinterpret_cast<const void *>(rotate_mma_kernel<R, true>), smem);
+  const long long nblk = (npoints + 63) / 64;
+  INQB_REQUIRE(nblk < (1LL << 31), INQB_ERR_UNSUPPORTED, "set too large for the rotation grid");
+  rotate_mma_kernel<R, true><<<unsigned(nblk), 128, smem, ctx.stream>>>(
+      phi, S, phi, S, npoints, X, make_double2(1.0, 0.0), make_double2(0.0, 0.0), 0, 0, skip_dev);
+  LAUNCHED(ctx);
+}
+
 template <typename R> void launch_rotate(Ctx &ctx, C2<R> *phi, int S, long long npoints, const double2 *Rdev) {
   launch_rotate_to<R>(ctx, phi, S, phi, S, npoints, Rdev, make_double2(1.0, 0.0), make_double2(0.0, 0.0));
 }
 
 // ------------------------------------------------------------------ density n[p] (+)= sum_s occ_s |phi[p][s]|^2
-// one warp per point, lanes stride over states, fixed shuffle tree (density.hpp:24-36)
-template <typename R>
+// One group of SL lanes per point (a warp, or as many lanes as the states below 32), lanes stride over the states,
+// fixed shuffle tree (density.hpp:24-36)
+template <typename R, int SL>
 __global__ void density_kernel(const C2<R> *__restrict__ phi, int S, long long npoints, const double *__restrict__ occ,
                                double *dens, int accumulate) {
-  const int lane = threadIdx.x & 31;
-  const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long p = warp; p < npoints; p += nwarps) {
+  const int lane = threadIdx.x % SL;
+  const long long group = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / SL;
+  const long long ngroups = ((long long)gridDim.x * blockDim.x) / SL;
+  // every lane of a warp runs the same number of rounds (the shuffles name the whole warp)
+  for (long long p0 = 0; p0 < npoints; p0 += ngroups) {
+    const long long p = p0 + group;
     double acc = 0.0;
-    for (int s = lane; s < S; s += 32) {
-      C2<R> x = phi[p * S + s];
-      acc += occ[s] * (double(x.x) * double(x.x) + double(x.y) * double(x.y));
+    if (p < npoints) {
+      for (int s = lane; s < S; s += SL) {
+        C2<R> x = phi[p * S + s];
+        acc += occ[s] * (double(x.x) * double(x.x) + double(x.y) * double(x.y));
+      }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) dens[p] = accumulate ? dens[p] + acc : acc;
+    for (int o = SL / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0 && p < npoints) dens[p] = accumulate ? dens[p] + acc : acc;
   }
 }
 template <typename R>
 void launch_density(Ctx &ctx, const C2<R> *phi, int S, long long npoints, const double *occ_dev, double *dens,
                     int accumulate) {
-  density_kernel<R><<<grid_for(npoints * 32, 256), 256, 0, ctx.stream>>>(phi, S, npoints, occ_dev, dens, accumulate);
-  LAUNCHED(ctx);
+  auto go = [&](auto kern, int sl) {
+    kern<<<grid_for(npoints * sl, 256), 256, 0, ctx.stream>>>(phi, S, npoints, occ_dev, dens, accumulate);
+    LAUNCHED(ctx);
+  };
+  if (S > 16) go(density_kernel<R, 32>, 32);
+  else if (S > 8) go(density_kernel<R, 16>, 16);
+  else if (S > 4) go(density_kernel<R, 8>, 8);
+  else go(density_kernel<R, 4>, 4);
 }
 
 // ------------------------------------------------------------------ kick: phi *= exp(i E_cov . r_contra)
@@ -1686,7 +1612,27 @@ template <typename R> void launch_kick(Ctx &ctx, const Basis &b, C2<R> *phi, int
   LAUNCHED(ctx);
 }
 
-// ------------------------------------------------------------------ sum |a - b| (integral_sum_absdiff)
+// ------------------------------------------------------------------ sums over a density
+constexpr int RED_BLOCKS = 592;  // block partials: 256 threads, four blocks per SM
+// out[c] = scale * sum of partial[b * nc + c] over the blocks b, nc <= 3 values, in a fixed order: one block,
+// each thread its strided share, then a tree (one thread adding all partials took 13 to 20 us)
+__global__ void __launch_bounds__(256) block_sums_kernel(const double *partial, int nb, int nc, double scale, double *out) {
+  __shared__ double red[256];
+  for (int c = 0; c < nc; c++) {
+    double acc = 0.0;
+    for (int b = threadIdx.x; b < nb; b += 256) acc += partial[b * nc + c];
+    red[threadIdx.x] = acc;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+      if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) out[c] = scale * red[0];
+    __syncthreads();
+  }
+}
+
+// sum |a - b| (integral_sum_absdiff)
 __global__ void absdiff_kernel(const double *a, const double *b, long long n, double *partial) {
   __shared__ double red[256];
   const long long chunk = (n + gridDim.x - 1) / gridDim.x;
@@ -1701,18 +1647,11 @@ __global__ void absdiff_kernel(const double *a, const double *b, long long n, do
   }
   if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
 }
-__global__ void absdiff_final_kernel(const double *partial, int nb, double *out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < nb; i++) s += partial[i];
-    *out = s;
-  }
-}
 void launch_absdiff_sum(Ctx &ctx, const double *a, const double *b, long long n, double *out_dev) {
   double *partial = static_cast<double *>(dev_alloc(ctx, sizeof(double) * RED_BLOCKS));
   absdiff_kernel<<<RED_BLOCKS, 256, 0, ctx.stream>>>(a, b, n, partial);
   LAUNCHED(ctx);
-  absdiff_final_kernel<<<1, 32, 0, ctx.stream>>>(partial, RED_BLOCKS, out_dev);
+  block_sums_kernel<<<1, 256, 0, ctx.stream>>>(partial, RED_BLOCKS, 1, 1.0, out_dev);
   LAUNCHED(ctx);
   dev_free(ctx, partial);
 }
@@ -1745,13 +1684,6 @@ __global__ void dipole_kernel(const double *__restrict__ dens, int nx, int ny, i
   }
   if (threadIdx.x < 3) partial[blockIdx.x * 3 + threadIdx.x] = red[threadIdx.x][0];
 }
-__global__ void dipole_final_kernel(const double *partial, int nb, double scale, double *out) {
-  if (blockIdx.x == 0 && threadIdx.x < 3) {
-    double s = 0.0;
-    for (int i = 0; i < nb; i++) s += partial[i * 3 + threadIdx.x];
-    out[threadIdx.x] = scale * s;
-  }
-}
 void launch_dipole(Ctx &ctx, const Basis &b, const double *dens, double *out3_dev) {
   double *partial = static_cast<double *>(dev_alloc(ctx, sizeof(double) * 3 * RED_BLOCKS));
   Vec3 a[3];
@@ -1759,7 +1691,7 @@ void launch_dipole(Ctx &ctx, const Basis &b, const double *dens, double *out3_de
     for (int j = 0; j < 3; j++) a[i].v[j] = b.lat[i][j];
   dipole_kernel<<<RED_BLOCKS, 256, 0, ctx.stream>>>(dens, b.n[0], b.n[1], b.n[2], b.npoints, a[0], a[1], a[2], partial);
   LAUNCHED(ctx);
-  dipole_final_kernel<<<1, 32, 0, ctx.stream>>>(partial, RED_BLOCKS, b.volume / double(b.npoints), out3_dev);
+  block_sums_kernel<<<1, 256, 0, ctx.stream>>>(partial, RED_BLOCKS, 3, b.volume / double(b.npoints), out3_dev);
   LAUNCHED(ctx);
   dev_free(ctx, partial);
 }
@@ -1780,27 +1712,6 @@ template <typename R>
 void launch_shift_cvec(Ctx &ctx, C2<R> *y, const C2<R> *x, int S, long long npoints, const double2 *coef_dev,
                        double scale) {
   shift_cvec_kernel<R><<<grid_for(npoints * S, 256), 256, 0, ctx.stream>>>(y, x, S, npoints * S, coef_dev, scale);
-  LAUNCHED(ctx);
-}
-
-// Teter-Payne-Allan preconditioner on a Fourier-space set (preconditioner.hpp:24-46):
-// x[G][s] *= K(0.5 |G|^2 / kin[s]), K(t) = (((8t + 12)t + 18)t + 27) / ((((16t + 8)t + 12)t + 18)t + 27)
-template <typename R>
-__global__ void tpa_precondition_kernel(Metric m, C2<R> *__restrict__ x, int S, long long n,
-                                        const double *__restrict__ kin) {
-  const double zero[3] = {0.0, 0.0, 0.0};
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double lapl = -0.5 * lapl_at(m, i / S, 1.0, zero, 0.0);  // -0.5 * (-|G|^2)
-    const double t = lapl / kin[i % S];
-    const double num = ((8.0 * t + 12.0) * t + 18.0) * t + 27.0;
-    const double den = (((16.0 * t + 8.0) * t + 12.0) * t + 18.0) * t + 27.0;
-    const double k = num / den;
-    x[i] = mk<C2<R>>(R(double(x[i].x) * k), R(double(x[i].y) * k));
-  }
-}
-template <typename R> void launch_tpa_precondition(Ctx &ctx, const Basis &b, C2<R> *x, int S, const double *kin_dev) {
-  tpa_precondition_kernel<R><<<grid_for(b.npoints * S, 256), 256, 0, ctx.stream>>>(metric_of(b), x, S,
-                                                                                   b.npoints * S, kin_dev);
   LAUNCHED(ctx);
 }
 
@@ -1996,15 +1907,10 @@ void launch_taylor_combine(Ctx &ctx, const C2<R> *x, const C2<R> *const *u, int 
   template void launch_shift_cvec<R>(Ctx &, C2<R> *, const C2<R> *, int, long long, const double2 *, double);      \
   template void launch_extract_states<R>(Ctx &, const C2<R> *, int, long long, int, int, double2 *);               \
   template void launch_insert_states<R>(Ctx &, const double2 *, int, long long, int, int, C2<R> *);                \
-  template void launch_tpa_precondition<R>(Ctx &, const Basis &, C2<R> *, int, const double *);                    \
   template void launch_laplacian<R>(Ctx &, const Basis &, const C2<R> *, C2<R> *, int, double, const double *);    \
-  template void launch_overlap_diag<R>(Ctx &, const C2<R> *, const C2<R> *, int, long long, double, double2 *);    \
-  template void launch_eigen_sums<R>(Ctx &, const C2<R> *, const C2<R> *, int, long long, double, double2 *,      \
-                                     double2 *);                                                                   \
-  template void launch_kinetic_ev<R>(Ctx &, const Basis &, const C2<R> *, int, double, const double *, double,     \
-                                     double *);                                                                   \
   template void launch_overlap<R>(Ctx &, const C2<R> *, int, const C2<R> *, int, long long, double, double2 *);   \
   template void launch_rotate<R>(Ctx &, C2<R> *, int, long long, const double2 *);                                 \
+  template void launch_rotate_upper<R>(Ctx &, C2<R> *, int, long long, const double2 *, const int *);              \
   template void launch_rotate_to<R>(Ctx &, const C2<R> *, int, C2<R> *, int, long long, const double2 *, double2,     \
                                     double2);                                                                      \
   template void launch_density<R>(Ctx &, const C2<R> *, int, long long, const double *, double *, int);            \

@@ -1,0 +1,104 @@
+"""Cholesky, triangular inverse, Jacobi rotations and per-state sums on the device, at state counts around the
+edges of their tiles, lane groups and clusters, against numpy and the host routines."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+EPS = 2.2e-16
+
+
+def _set(nst, sizes=(12, 10, 9), seed=0, precision=None):
+    import inq_b200 as ib
+    rng = np.random.default_rng(seed + nst)
+    basis = ib.RealSpace(ib.Cell.orthorhombic(*[0.5 * n for n in sizes]), sizes=sizes)
+    x = rng.standard_normal((basis.size(), nst)) + 1j * rng.standard_normal((basis.size(), nst))
+    return basis, rng, x, ib.OrbitalSet.from_array(basis, x, precision=ib.F64 if precision is None else precision)
+
+
+# phi U^-1 against numpy's factor: the overlaps of random sets have condition numbers below 1e3 here (fewer
+# states than half the points), which with sums of 1080 terms leaves about 1e3 * 30 * EPS
+@pytest.mark.parametrize("nst", [1, 2, 31, 32, 33, 64, 65, 100, 129, 200, 257, 400])
+def test_orthogonalize(nst):
+    import inq_b200 as ib
+    basis, _, x, phi = _set(nst)
+    dv = basis.volume_element()
+    ref = x @ np.linalg.inv(np.linalg.cholesky(dv * (x.conj().T @ x)).conj().T)
+    ib.orthogonalize(phi)
+    got = phi.matrix()
+    assert np.linalg.norm(got - ref) < 1e-11 * np.linalg.norm(ref)
+    S = dv * (got.conj().T @ got)
+    assert np.abs(S - np.eye(nst)).max() < 1e-12
+
+
+@pytest.mark.parametrize("nst", [5, 33, 64, 65])
+def test_orthogonalize_single(nst):
+    import inq_b200 as ib
+    basis, _, x, phi = _set(nst, precision=ib.F32)
+    ib.orthogonalize(phi)
+    got = phi.matrix().astype(complex)
+    S = basis.volume_element() * (got.conj().T @ got)
+    assert np.abs(S - np.eye(nst)).max() < 1e-5  # split-BF16 overlaps: 1e-6 per element times the condition number
+
+
+@pytest.mark.parametrize("nst", [3, 40])
+def test_orthogonalize_refuses_dependent_states(nst):
+    import inq_b200 as ib
+    _, _, x, _ = _set(nst)
+    x[:, nst - 1] = 0.0
+    basis, _, _, phi = _set(nst)
+    phi.upload(x)
+    with pytest.raises(ib.InqbError, match="not positive definite"):
+        ib.orthogonalize(phi)
+    assert np.array_equal(phi.matrix(), x)
+
+
+# The device's waves are the host routine's rotations in another order of independent ones: eigenvalues agree
+# to rounding, eigenvectors to rounding over the smallest gap, each up to a phase.  The phase of a vector is
+# that of the off-diagonal element r of its last rotation by about pi / 2 (which swaps two columns), known to
+# EPS * norm / r: dense random matrices still swap columns at r = 1e-10 norm and below, so for them the phases
+# hold to 1e-3 only (5e-6 seen at 130 states; the host routine moves as much when a last bit of H changes).
+@pytest.mark.parametrize("nst", [1, 2, 13, 14, 15, 64, 97, 130])
+def test_subspace_diagonalization_matches_host_rotations(nst):
+    import inq_b200 as ib
+    basis, rng, x, phi = _set(nst)
+    ham = ib.KSHamiltonian(basis)
+    ham.set_scalar_potential(rng.standard_normal(basis.sizes))
+    ib.orthogonalize(phi)
+    H = ib.overlap(phi, ham(phi))
+    w, V = ib.hermitian_eigen(H)
+    ref = phi.matrix() @ V
+    eig = ham.subspace_diagonalization(phi)
+    got = phi.matrix()
+    norm = np.abs(w).max()
+    assert np.all(np.diff(eig) >= 0.0)
+    assert np.abs(eig - w).max() < 100 * EPS * norm * max(1, nst) ** 0.5
+    gap = np.diff(w).min() if nst > 1 else norm
+    z = (ref.conj() * got).sum(0) / (np.abs(ref) ** 2).sum(0)
+    assert np.linalg.norm(got - ref * (z / np.abs(z))) < (1e-12 + 200 * EPS * norm / gap) * np.linalg.norm(ref)
+    assert np.abs(z - 1.0).max() < 1e-3
+
+
+# sums of npoints products in double (double of single-precision values): 1e-13 of the norms is 100 roundings
+@pytest.mark.parametrize("nst", [1, 7, 8, 9, 33, 128, 200, 256, 257, 300])
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+def test_state_sums(nst, precision):
+    import inq_b200 as ib
+    prec = ib.F64 if precision == "f64" else ib.F32
+    basis, rng, x, phi = _set(nst, sizes=(9, 7, 5), precision=prec)
+    a = phi.matrix().astype(complex)
+    b_set = ib.OrbitalSet.from_array(basis, x[::-1].copy(), precision=prec)
+    b = b_set.matrix().astype(complex)
+    dv = basis.volume_element()
+    scale = dv * np.sqrt((np.abs(a) ** 2).sum(0) * (np.abs(b) ** 2).sum(0))
+    assert np.all(np.abs(ib.overlap_diagonal(phi, b_set) - dv * (a.conj() * b).sum(0)) < 1e-13 * scale)
+    ham = ib.KSHamiltonian(basis)
+    ham.set_scalar_potential(rng.standard_normal(basis.sizes))
+    h = ham(phi).matrix().astype(complex)
+    n2 = (np.abs(a) ** 2).sum(0)
+    e = (a.conj() * h).real.sum(0) / n2
+    eig, res = ham.eigenvalues(phi)
+    assert np.all(np.abs(eig - e) < 1e-12 * np.abs(h).max())
+    assert np.allclose(res, dv * (np.abs(h - e * a) ** 2).sum(0), rtol=1e-11)
+    occ = rng.uniform(0.0, 2.0, nst)
+    dens = ib.density([phi, b_set], [occ, occ])
+    assert np.allclose(dens, (np.abs(a) ** 2) @ occ + (np.abs(b) ** 2) @ occ, rtol=1e-13)
