@@ -21,6 +21,7 @@
 
 #include "fft2_lengths.h"
 #include "fft_common.cuh"
+#include "ptx.cuh"
 
 namespace inqb {
 
@@ -44,6 +45,8 @@ __global__ void __launch_bounds__(256) fft_pass_kernel(PassArgs<R> a, Geom g, Ra
   const int s = s0 + w;
   const bool active = s < a.S;
   const int n = rad.n;
+  ptx::grid_wait();
+  ptx::grid_release();
 
   // ---- load (coalesced rows of W states)
   for (int p = jg; p < n; p += njg) {
@@ -135,8 +138,7 @@ void launch_fft_pass(Ctx &ctx, const Basis &b, const PassArgs<R> &a, int prologu
 
   auto go = [&](auto kern) {
     ensure_smem_attr(reinterpret_cast<const void *>(kern), smem);
-    kern<<<unsigned(tiles), threads, smem, ctx.stream>>>(a, g, rad, tw, W);
-    INQB_CUDA(cudaGetLastError());
+    pdl_launch(kern, dim3(unsigned(tiles)), threads, smem, ctx.stream, a, g, rad, tw, W);
     ctx.launches++;
   };
   if (prologue == PRO_NONE && epilogue == EPI_STORE) go(fft_pass_kernel<R, PRO_NONE, EPI_STORE>);

@@ -819,6 +819,8 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
     mbar_init_fence();
   }
   __syncthreads();
+  ptx::grid_wait();
+  ptx::grid_release();
 
   auto coords = [&](long long t, int &c0, int &c1, int &c2, int &c3) {
     if (gg.flat) {
@@ -1180,6 +1182,8 @@ __global__ void __launch_bounds__(zl_max_threads<R>()) fftz_kernel(PassArgs<R> a
     mbar_init_fence();
   }
   __syncthreads();
+  ptx::grid_wait();
+  ptx::grid_release();
 
   auto wait_bar = [&](uint64_t *b, uint32_t parity) -> bool {
     const uint64_t t0 = global_ns();
@@ -1487,8 +1491,7 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
     mb = (has_aux(VAR) && a.hbase) ? orbital_map(a.hbase, b, a.S, cwords, gg.axis, W) : mi;
   }
   const TC *tw = reinterpret_cast<const TC *>(sizeof(CR) == 8 ? b.tw64[gg.axis] : b.tw32[gg.axis]);
-  kern<<<unsigned(grid), NT, smem, ctx.stream>>>(mi, mo, mx, mb, a, gg, tw, ctx.d_err);
-  INQB_CUDA(cudaGetLastError());
+  pdl_launch(kern, dim3(unsigned(grid)), NT, smem, ctx.stream, mi, mo, mx, mb, a, gg, tw, ctx.d_err);
   ctx.launches++;
 }
 
@@ -1569,8 +1572,7 @@ void launch_zlines(Ctx &ctx, const Basis &b, const PassArgs<R> &a, const ZLines 
   long long grid = (long long)(ctas < 1 ? 1 : (ctas > 8 ? 8 : ctas)) * ctx.num_sms;
   if (grid > tiles) grid = tiles;
   const T *tw = reinterpret_cast<const T *>(sizeof(R) == 8 ? b.tw64[2] : b.tw32[2]);
-  kern<<<unsigned(grid), z.threads + 32, smem, ctx.stream>>>(a, gz, tw, ctx.d_err);
-  INQB_CUDA(cudaGetLastError());
+  pdl_launch(kern, dim3(unsigned(grid)), z.threads + 32, smem, ctx.stream, a, gz, tw, ctx.d_err);
   ctx.launches++;
 }
 

@@ -156,6 +156,8 @@ __global__ void __launch_bounds__(NLP_WARPS * 32) nl_project_kernel(const C2<R> 
   const int SL = 1 << sl, G = 32 >> sl;        // lanes per group, groups per warp
   const int ls = lane & (SL - 1), g = lane >> sl;
   const int sbase = blockIdx.z * SL * K;
+  ptx::grid_wait();
+  ptx::grid_release();
   const int np = npts[p];
   const int nr = int(gridDim.y);  // ranges of a sphere
   const int rper = (np + nr - 1) / nr;
@@ -248,12 +250,6 @@ __global__ void __launch_bounds__(NLA_NT + 32) nl_project_bulk_kernel(const C2<R
   uint64_t *full = reinterpret_cast<uint64_t *>(gs + size_t(NLP_NS) * KB * 4);  // stage loaded
   uint64_t *done = full + NLP_NS;                                            // stage consumed
   volatile int *abort_flag = reinterpret_cast<volatile int *>(done + NLP_NS);
-  const int np = npts[p];
-  const int nr = int(gridDim.y);  // ranges of a sphere
-  const int rper = (np + nr - 1) / nr;
-  const int r0 = rg * rper, r1 = min(np, r0 + rper);
-  const int n = max(r1 - r0, 0);
-  const int nbatch = (n + KB - 1) / KB;
   const long long rowbase = (long long)p * maxsph;
   const uint32_t row_bytes = uint32_t(SC) * uint32_t(sizeof(T));
   if (threadIdx.x == 0) {
@@ -265,6 +261,14 @@ __global__ void __launch_bounds__(NLA_NT + 32) nl_project_bulk_kernel(const C2<R
     mbar_init_fence();
   }
   __syncthreads();
+  grid_wait();
+  grid_release();
+  const int np = npts[p];
+  const int nr = int(gridDim.y);  // ranges of a sphere
+  const int rper = (np + nr - 1) / nr;
+  const int r0 = rg * rper, r1 = min(np, r0 + rper);
+  const int n = max(r1 - r0, 0);
+  const int nbatch = (n + KB - 1) / KB;
 
   if (threadIdx.x >= NLA_NT) {
     // producer warp: lane q copies point q of a batch, lane 0 also the batch's coefficients
@@ -364,6 +368,8 @@ __global__ void __launch_bounds__(NLF_S * 4) nl_project_finish_kernel(const C2<A
   __shared__ TA pr[4][NLF_S];
   const int p = blockIdx.x / nsb, l = threadIdx.x / NLF_S, c = threadIdx.x % NLF_S;
   const int s = (blockIdx.x % nsb) * NLF_S + c;
+  ptx::grid_wait();
+  ptx::grid_release();
   if (s < S) {
     const TA *src = partial + ((long long)p * nr * 4 + l) * S + s;
     const long long step = 4LL * S;
@@ -446,23 +452,23 @@ void launch_nl_project(Ctx &ctx, const Basis &b, const Hamiltonian &h, const C2<
       const size_t smem = smem_of(KB);
       auto kern = nl_project_bulk_kernel<R, A, JB>;
       ensure_smem_attr(reinterpret_cast<const void *>(kern), smem);
-      kern<<<dim3(P.nproj, NR, nchunks), NLA_NT + 32, smem, ctx.stream>>>(psi, S, P.d_pt, gcoef, P.d_npts, P.maxsph, KB,
-                                                                        part, ctx.d_err);
+      pdl_launch(kern, dim3(P.nproj, NR, nchunks), NLA_NT + 32, smem, ctx.stream, psi, S, P.d_pt, gcoef, P.d_npts, P.maxsph,
+                 KB, part, ctx.d_err);
     } else {
       const dim3 grid(P.nproj, NR, rchunks);
       // four points in flight at two states per lane (eight: 94 against 50 us at 72^3 x 99 single)
       if (K == 2)
-        nl_project_kernel<R, A, 2, 4><<<grid, NLP_WARPS * 32, 0, ctx.stream>>>(psi, S, sl, P.d_pt, gcoef, P.d_npts,
-                                                                                P.maxsph, part);
+        pdl_launch(nl_project_kernel<R, A, 2, 4>, grid, NLP_WARPS * 32, 0, ctx.stream, psi, S, sl, P.d_pt, gcoef, P.d_npts,
+                   P.maxsph, part);
       else
-        nl_project_kernel<R, A, 1, 8><<<grid, NLP_WARPS * 32, 0, ctx.stream>>>(psi, S, sl, P.d_pt, gcoef, P.d_npts,
-                                                                              P.maxsph, part);
+        pdl_launch(nl_project_kernel<R, A, 1, 8>, grid, NLP_WARPS * 32, 0, ctx.stream, psi, S, sl, P.d_pt, gcoef, P.d_npts,
+                   P.maxsph, part);
     }
-    LAUNCHED(ctx);
+    ctx.launches++;
     const int nsb = (S + NLF_S - 1) / NLF_S;
-    nl_project_finish_kernel<R, A><<<unsigned(P.nproj) * nsb, NLF_S * 4, 0, ctx.stream>>>(part, nsb, NR, S, coeff,
-                                                                                         projraw, projD);
-    LAUNCHED(ctx);
+    pdl_launch(nl_project_finish_kernel<R, A>, dim3(unsigned(P.nproj) * nsb), NLF_S * 4, 0, ctx.stream, part, nsb, NR, S,
+               coeff, projraw, projD);
+    ctx.launches++;
   };
   if (dbl) go(double());
   else go(float());
@@ -551,6 +557,8 @@ __global__ void __launch_bounds__(128) nl_apply_kernel(NlApply<R> a, long long n
   const int ls = threadIdx.x & (SL - 1);
   const long long group = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> sl;
   const long long ngroups = ((long long)gridDim.x * blockDim.x) >> sl;
+  ptx::grid_wait();
+  ptx::grid_release();
   // the record of the group's next item is requested while the current one is processed
   int4 next = group < nitems ? a.hrec[group / nchunks] : make_int4(0, 0, 0, 0);
   for (long long it = group; it < nitems; it += ngroups) {
@@ -617,6 +625,8 @@ __global__ void __launch_bounds__(NLA_NT + 32, sizeof(R) == 4 ? 6 : 3) nl_apply_
     mbar_init_fence();
   }
   __syncthreads();
+  grid_wait();
+  grid_release();
   auto wait_bar = [&](uint64_t *b, uint32_t parity) { return nla_wait(b, parity, abort_flag, err); };
 
   if (threadIdx.x >= NLA_NT) {
@@ -778,8 +788,8 @@ void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, 
       const long long nbatch = (P.nhitpts + KB - 1) / KB;
       long long grid = (long long)(per_sm < 1 ? 1 : per_sm) * ctx.num_sms;
       if (grid > nbatch) grid = nbatch;
-      kern<<<unsigned(grid), NLA_NT + 32, smem, ctx.stream>>>(a, P.nhitpts, KB, ts, ctx.d_err);
-      LAUNCHED(ctx);
+      pdl_launch(kern, dim3(unsigned(grid)), NLA_NT + 32, smem, ctx.stream, a, P.nhitpts, KB, ts, ctx.d_err);
+      ctx.launches++;
       return;
     }
   }
@@ -794,8 +804,8 @@ void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, 
   using Kern = void (*)(NlApply<R>, long long, int, int);
   const Kern kern = S <= 32 ? (V ? Kern(nl_apply_kernel<R, 1, true>) : Kern(nl_apply_kernel<R, 1, false>))
                             : (V ? Kern(nl_apply_kernel<R, U, true>) : Kern(nl_apply_kernel<R, U, false>));
-  kern<<<unsigned(blocks), 128, 0, ctx.stream>>>(a, nitems, nchunks, sl);
-  LAUNCHED(ctx);
+  pdl_launch(kern, dim3(unsigned(blocks)), 128, 0, ctx.stream, a, nitems, nchunks, sl);
+  ctx.launches++;
 }
 
 // ------------------------------------------------------------------ bounded-wait self-test

@@ -35,6 +35,15 @@ __device__ __forceinline__ uint64_t global_ns() {
 // generic-proxy shared-memory writes made visible to the async proxy (TMA, tensor cores)
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+
+// A kernel launched by pdl_launch may start while its predecessor in the stream still runs: it may set up
+// shared memory, barriers and constant tables first, and must wait here before it touches anything else in
+// global memory.  Every thread of every kernel launched that way calls it.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the next kernel of the stream may start (once every CTA has said so or ended)
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- bulk asynchronous copies (TMA engine)
 
 // arrive on `bar` and expect `bytes` more transaction bytes in its current phase
