@@ -138,7 +138,7 @@ void launch_fft_pass(Ctx &ctx, const Basis &b, const PassArgs<R> &a, int prologu
 
   auto go = [&](auto kern) {
     ensure_smem_attr(reinterpret_cast<const void *>(kern), smem);
-    pdl_launch(kern, dim3(unsigned(tiles)), threads, smem, ctx.stream, a, g, rad, tw, W);
+    pdl_launch(true, kern, dim3(unsigned(tiles)), threads, smem, ctx.stream, a, g, rad, tw, W);
     ctx.launches++;
   };
   if (prologue == PRO_NONE && epilogue == EPI_STORE) go(fft_pass_kernel<R, PRO_NONE, EPI_STORE>);

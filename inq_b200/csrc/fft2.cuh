@@ -946,6 +946,26 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
     if (blockIdx.x < gg.ntiles) cpa_load_stage(0, blockIdx.x);
     ptx::cp_async_commit();
   }
+  // V of a tile's line: in double requested one tile ahead (raw, so that nothing waits for it before the next
+  // tile; 120^3 x 64 final pass 872 -> 826 us); single-precision passes lose by it (96^3 x 256 816 -> 877)
+  constexpr bool LINEV = base_var(VAR) == INV_FINAL || VAR == FWD_VPSI;
+  constexpr bool AHEAD = LINEV && sizeof(R) == 8;
+  constexpr int VB = LINEV ? (N + NT - 1) / NT : 1;
+  R nextv[VB];
+  int nexth[VAR == FWD_VPSI ? VB : 1];  // sphere hits of the point
+  auto request_v = [&](long long t) {
+    if constexpr (LINEV) {
+      const long long L = t / gg.nsb, pb = (L / g.nb) * g.sa + (L % g.nb) * g.sb;
+#pragma unroll
+      for (int k = 0; k < VB; k++) {
+        const int m = threadIdx.x + k * NT;
+        const long long pt = pb + (m < N ? m : 0) * g.sp;
+        nextv[k] = a.V[pt * a.nspin + a.spin];
+        if constexpr (VAR == FWD_VPSI) nexth[k] = a.nl_offs ? a.nl_offs[pt + 1] - a.nl_offs[pt] : 0;
+      }
+    }
+  };
+  if (AHEAD && blockIdx.x < gg.ntiles) request_v(blockIdx.x);
   int i = 0;
   for (long long t = blockIdx.x; t < gg.ntiles; t += gridDim.x, i++) {
     const int st = i % NS;
@@ -1011,10 +1031,19 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
         if (a.perm_n2[2]) iz = iz / a.perm_n2[2] + (g.n[2] / a.perm_n2[2]) * (iz % a.perm_n2[2]);
         linev[m] = CR(lapl_value(g, ix, iy, iz, a.lap_factor, a.gc));
       }
-    } else if constexpr (base_var(VAR) == INV_FINAL || VAR == FWD_VPSI) {
+    } else if constexpr (AHEAD) {
+#pragma unroll
+      for (int k = 0; k < VB; k++) {
+        const int m = threadIdx.x + k * NT;
+        // Fourier form: points with sphere hits already hold (V + shift) psi + nonlocal
+        bool masked = false;
+        if constexpr (VAR == FWD_VPSI) masked = nexth[k] > 0;
+        if (m < N) linev[m] = masked ? CR(1) : CR(nextv[k]) + CR(a.vshift);
+      }
+      if (t + gridDim.x < gg.ntiles) request_v(t + gridDim.x);
+    } else if constexpr (LINEV) {
       for (int m = threadIdx.x; m < N; m += NT) {
         const long long pt = pbase + m * g.sp;
-        // Fourier form: points with sphere hits already hold (V + shift) psi + nonlocal
         const bool masked = VAR == FWD_VPSI && a.nl_offs && a.nl_offs[pt + 1] > a.nl_offs[pt];
         linev[m] = masked ? CR(1) : CR(a.V[pt * a.nspin + a.spin]) + CR(a.vshift);
       }
@@ -1232,6 +1261,23 @@ __global__ void __launch_bounds__(zl_max_threads<R>()) fftz_kernel(PassArgs<R> a
   const bool horner = FINAL && a.hbase != nullptr;
   const bool scaled = a.scale != 1.0;
   const int tid = threadIdx.x, colS = N2 * S, rowS = N1 * S;
+  // V of the chunk's point tid: in double requested one chunk ahead
+  constexpr bool AHEAD = LINEV && sizeof(R) == 8;
+  // psi of an item of the last step one item ahead: in double (54 x 60 x 45 x 50 87 -> 76 us) while the registers
+  // last (80^3 x 40: H 717 -> 765 us with spills); single precision loses by it (72^3 x 99 181 -> 199 us)
+  constexpr bool PSI_AHEAD = FINAL && sizeof(R) == 8 && N1 + N2 <= 16;
+  R nextv = R(0);
+  int nexth = 0;
+  auto request_v = [&](int t) {
+    if constexpr (LINEV) {
+      const long long pt = (long long)t * gz.lpt * N + tid;
+      if (tid < lines_of(t) * N) {
+        nextv = a.V[pt * a.nspin + a.spin];
+        if (VAR == FWD_VPSI && a.nl_offs) nexth = a.nl_offs[pt + 1] - a.nl_offs[pt];
+      }
+    }
+  };
+  if (AHEAD && int(blockIdx.x) < gz.ntiles) request_v(blockIdx.x);
   int i = 0;
   for (int t = blockIdx.x; t < gz.ntiles; t += gridDim.x, i++) {
     const int st = i % NS;
@@ -1243,17 +1289,32 @@ __global__ void __launch_bounds__(zl_max_threads<R>()) fftz_kernel(PassArgs<R> a
     T *__restrict__ out = a.out + g0;
     if constexpr (LINEV) {
       const long long p0 = (long long)t * gz.lpt * N;
-      const bool masked = VAR == FWD_VPSI && a.nl_offs != nullptr;
-      for (int m = tid; m < nl * N; m += NT) {
+      const bool hits = VAR == FWD_VPSI && a.nl_offs != nullptr;
+      // points with sphere hits already hold (V + shift) psi + nonlocal
+      if (AHEAD && tid < nl * N) linev[tid] = hits && nexth > 0 ? R(1) : nextv + a.vshift;
+      for (int m = AHEAD ? tid + NT : tid; m < nl * N; m += NT) {
         const long long pt = p0 + m;
-        // points with sphere hits already hold (V + shift) psi + nonlocal
-        linev[m] = masked && a.nl_offs[pt + 1] > a.nl_offs[pt] ? R(1) : a.V[pt * a.nspin + a.spin] + a.vshift;
+        linev[m] = hits && a.nl_offs[pt + 1] > a.nl_offs[pt] ? R(1) : a.V[pt * a.nspin + a.spin] + a.vshift;
       }
+      if (AHEAD && t + int(gridDim.x) < gz.ntiles) request_v(t + gridDim.x);
       if constexpr (VAR == FWD_VPSI) sync();
     }
 
     if constexpr (VAR == INV_PERM || VAR == INV_FINAL_PERM) {
-      // rows first (digit-reversed input), then columns in natural order
+      // rows first (digit-reversed input), then columns in natural order; the first column item's psi is
+      // requested before the rows, each further one an item ahead
+      T xn[PSI_AHEAD ? N1 : 1];
+      auto request_psi = [&](int it) {
+        if constexpr (PSI_AHEAD) {
+          if (it < nl * colS) {
+            const int l = nl > 1 ? div_by(it, gz.mag_a) : 0;
+            const T *src = a.psi + g0 + it + (long long)l * (line - colS);
+#pragma unroll
+            for (int j1 = 0; j1 < N1; j1++) xn[j1] = src[j1 * colS];
+          }
+        }
+      };
+      request_psi(tid);
       for (int it = tid; it < nl * rowS; it += NT) {
         const int l = nl > 1 ? div_by(it, gz.mag_b) : 0, r = it - l * rowS;
         const int k1 = div_by(r, gz.mag_s);
@@ -1276,7 +1337,8 @@ __global__ void __launch_bounds__(zl_max_threads<R>()) fftz_kernel(PassArgs<R> a
         T x[FINAL ? N1 : 1], h[FINAL ? N1 : 1];
         if constexpr (FINAL) {
 #pragma unroll
-          for (int j1 = 0; j1 < N1; j1++) x[j1] = a.psi[g0 + e0 + j1 * colS];
+          for (int j1 = 0; j1 < N1; j1++) x[j1] = PSI_AHEAD ? xn[PSI_AHEAD ? j1 : 0] : a.psi[g0 + e0 + j1 * colS];
+          request_psi(it + NT);  // the next item's, while this one is transformed
           if (horner) {
 #pragma unroll
             for (int j1 = 0; j1 < N1; j1++) h[j1] = a.hbase[g0 + e0 + j1 * colS];
@@ -1427,13 +1489,6 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
   gg.flines = ((VAR == MID_KIN || VAR == FWD_LAPLADD) && gg.flat && a.S < W) ? ((W - 1) / a.S + 3) / 2 * 2 : 2;
   const size_t fixed = (SPLIT ? size_t(N) * W * sizeof(TC) : 0) + size_t(tw_entries<CR>(N)) * sizeof(TC) +
                        size_t(gg.flines) * N * sizeof(CR) + 64 + 16 * 8;
-  // shared memory per CTA: ~113 KB (two CTAs per SM) for the FP64 streaming passes; ~56 KB (four per SM)
-  // for the wide-arithmetic, the kinetic and the producer-warp (single-precision) passes, whose
-  // arithmetic needs more warps to hide latency (96^3 x 256 single: 3.81 ms per H against 3.89 with
-  // four stages of 113 KB)
-  size_t budget = (SPLIT || VAR == MID_KIN || ws_of<R, CR, N, VAR>()) ? 56 * 1024 : 113 * 1024;
-  // 512-byte-row streaming passes: three stages, one CTA per SM
-  if (WIDE) budget = 150 * 1024;
   // second input tiles beside every ring stage when two stages of them leave room for two CTAs per SM,
   // else single-buffered (96^3 x 256: 0.80 against 0.92 ms for the single-precision final pass beside
   // every stage; 120^3 x 256 double: 3.1 against 5.35 ms single-buffered, at two CTAs per SM against one)
@@ -1441,8 +1496,37 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
   gg.aux_single = !gg.cpa && naux > 0 && size_t(2) * (1 + naux) * TILE_BYTES + fixed > 113 * 1024;
   const size_t per_stage = TILE_BYTES * (gg.aux_single ? 1 : 1 + naux);
   const size_t fixed_aux = gg.aux_single ? naux * TILE_BYTES : 0;
-  int ns = budget > fixed + fixed_aux ? int((budget - fixed - fixed_aux) / per_stage) : 0;
-  ns = ns < 2 ? 2 : (ns > 6 ? 6 : ns);
+  // Ring depth.  What counts is the warps per SM that cover the arithmetic's latency, then the bytes in flight;
+  // measured per pass (us, one transit in and out at 6.4 TB/s in brackets):
+  //  * double: two stages, so that four to six CTAs share an SM (fwd/inv y pass 60^3 x 64 95/98 -> 81/74 [69],
+  //    120^3 x 64 630/622 -> 576/564 [549]; final pass, two tiles per stage, 64^3 x 128 345 -> 252, 48^3 x 128
+  //    183 -> 113); three in the streaming passes of lines with one first-step item per thread (64, 96 and 128
+  //    points: 96^3 x 128 554/547 with three, 604/597 with two), and in their kinetic pass of sets beyond L2;
+  //  * single, 512-byte rows: three stages for sets that stay in L2 (two to three CTAs per SM up to 72 points:
+  //    48^3 x 97 37/36 with six stages, 26/24 with three [27]), four for larger ones while they fit 150 KB
+  //    (72^3 x 250 276/269 with three, 240/248 with four [232]), three up to 204 KB (120^3 x 64 350/336 with
+  //    two, 274/286 with three [274]); two where the steps leave part of the CTA idle in their last round
+  //    (N1 no multiple of 4: 90^3 x 128 255/270 with three, 244/244 with two [232]);
+  //  * other single-precision passes and wider arithmetic: about 56 KB per CTA (four per SM), two stages for sets
+  //    that stay in L2 (as fast alone, and the CTAs find room beside the previous pass's last ones).
+  constexpr int NTC = threads_of<R, CR, N, VAR, WIDE>();
+  const bool in_l2 = size_t(b.npoints) * a.S * sizeof(T) <= (size_t(128) << 20);
+  auto bytes = [&](int n) { return per_stage * n + fixed_aux + fixed; };
+  int ns;
+  if (WIDE) {
+    if ((W * Split<N>::N1) % NTC != 0 && bytes(2) <= 110 * 1024) ns = 2;
+    else {
+      ns = in_l2 ? 3 : 4;
+      if (ns == 4 && bytes(4) > 150 * 1024) ns = 3;
+      if (ns == 3 && bytes(3) > 204 * 1024) ns = 2;
+    }
+  } else if (sizeof(R) == 8) {
+    constexpr bool exact = W * Split<N>::N2 == NTC;
+    ns = naux == 0 && exact && (VAR != MID_KIN || !in_l2) ? 3 : 2;
+  } else {
+    ns = 56 * 1024 > fixed + fixed_aux ? int((56 * 1024 - fixed - fixed_aux) / per_stage) : 0;
+    ns = ns < 2 || in_l2 ? 2 : (ns > 6 ? 6 : ns);
+  }
   if (ctx.fft_stages > 0) ns = ctx.fft_stages < 2 ? 2 : ctx.fft_stages;
   if (gg.cpa) ns = 2;
   gg.stages = ns;
@@ -1491,7 +1575,10 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
     mb = (has_aux(VAR) && a.hbase) ? orbital_map(a.hbase, b, a.S, cwords, gg.axis, W) : mi;
   }
   const TC *tw = reinterpret_cast<const TC *>(sizeof(CR) == 8 ? b.tw64[gg.axis] : b.tw32[gg.axis]);
-  pdl_launch(kern, dim3(unsigned(grid)), NT, smem, ctx.stream, mi, mo, mx, mb, a, gg, tw, ctx.d_err);
+  // sets beyond L2 start their passes the ordinary way: CTAs that come early settle unevenly in the room the
+  // previous pass leaves, and these passes are long enough for that to cost more than the launch gap (H at
+  // 64^3 x 128 FP64 1202 -> 1072 us, 96^3 x 120 single 1625 -> 1592, 96^3 x 256 single 3492 -> 3456)
+  pdl_launch(in_l2, kern, dim3(unsigned(grid)), NT, smem, ctx.stream, mi, mo, mx, mb, a, gg, tw, ctx.d_err);
   ctx.launches++;
 }
 
@@ -1572,7 +1659,7 @@ void launch_zlines(Ctx &ctx, const Basis &b, const PassArgs<R> &a, const ZLines 
   long long grid = (long long)(ctas < 1 ? 1 : (ctas > 8 ? 8 : ctas)) * ctx.num_sms;
   if (grid > tiles) grid = tiles;
   const T *tw = reinterpret_cast<const T *>(sizeof(R) == 8 ? b.tw64[2] : b.tw32[2]);
-  pdl_launch(kern, dim3(unsigned(grid)), z.threads + 32, smem, ctx.stream, a, gz, tw, ctx.d_err);
+  pdl_launch(true, kern, dim3(unsigned(grid)), z.threads + 32, smem, ctx.stream, a, gz, tw, ctx.d_err);
   ctx.launches++;
 }
 

@@ -189,7 +189,7 @@ struct Hamiltonian {
 // kernels take themselves.  Measured with against without: H at 24^3 x 9 single 27 against 45 us, 32^3 x 16
 // FP64 56 against 75, 64^3 x 64 single 296 against 314, 72^3 x 99 single 725 against 732.
 template <typename... KA, typename... A>
-void pdl_launch(void (*kern)(KA...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A &&...args) {
+void pdl_launch(bool early, void (*kern)(KA...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A &&...args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -199,7 +199,7 @@ void pdl_launch(void (*kern)(KA...), dim3 grid, unsigned threads, size_t smem, c
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;  // 0: an ordinary launch, for which grid_wait() returns at once
   INQB_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...));
 }
 

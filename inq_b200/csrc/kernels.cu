@@ -452,21 +452,21 @@ void launch_nl_project(Ctx &ctx, const Basis &b, const Hamiltonian &h, const C2<
       const size_t smem = smem_of(KB);
       auto kern = nl_project_bulk_kernel<R, A, JB>;
       ensure_smem_attr(reinterpret_cast<const void *>(kern), smem);
-      pdl_launch(kern, dim3(P.nproj, NR, nchunks), NLA_NT + 32, smem, ctx.stream, psi, S, P.d_pt, gcoef, P.d_npts, P.maxsph,
+      pdl_launch(true, kern, dim3(P.nproj, NR, nchunks), NLA_NT + 32, smem, ctx.stream, psi, S, P.d_pt, gcoef, P.d_npts, P.maxsph,
                  KB, part, ctx.d_err);
     } else {
       const dim3 grid(P.nproj, NR, rchunks);
       // four points in flight at two states per lane (eight: 94 against 50 us at 72^3 x 99 single)
       if (K == 2)
-        pdl_launch(nl_project_kernel<R, A, 2, 4>, grid, NLP_WARPS * 32, 0, ctx.stream, psi, S, sl, P.d_pt, gcoef, P.d_npts,
+        pdl_launch(true, nl_project_kernel<R, A, 2, 4>, grid, NLP_WARPS * 32, 0, ctx.stream, psi, S, sl, P.d_pt, gcoef, P.d_npts,
                    P.maxsph, part);
       else
-        pdl_launch(nl_project_kernel<R, A, 1, 8>, grid, NLP_WARPS * 32, 0, ctx.stream, psi, S, sl, P.d_pt, gcoef, P.d_npts,
+        pdl_launch(true, nl_project_kernel<R, A, 1, 8>, grid, NLP_WARPS * 32, 0, ctx.stream, psi, S, sl, P.d_pt, gcoef, P.d_npts,
                    P.maxsph, part);
     }
     ctx.launches++;
     const int nsb = (S + NLF_S - 1) / NLF_S;
-    pdl_launch(nl_project_finish_kernel<R, A>, dim3(unsigned(P.nproj) * nsb), NLF_S * 4, 0, ctx.stream, part, nsb, NR, S,
+    pdl_launch(true, nl_project_finish_kernel<R, A>, dim3(unsigned(P.nproj) * nsb), NLF_S * 4, 0, ctx.stream, part, nsb, NR, S,
                coeff, projraw, projD);
     ctx.launches++;
   };
@@ -788,7 +788,7 @@ void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, 
       const long long nbatch = (P.nhitpts + KB - 1) / KB;
       long long grid = (long long)(per_sm < 1 ? 1 : per_sm) * ctx.num_sms;
       if (grid > nbatch) grid = nbatch;
-      pdl_launch(kern, dim3(unsigned(grid)), NLA_NT + 32, smem, ctx.stream, a, P.nhitpts, KB, ts, ctx.d_err);
+      pdl_launch(true, kern, dim3(unsigned(grid)), NLA_NT + 32, smem, ctx.stream, a, P.nhitpts, KB, ts, ctx.d_err);
       ctx.launches++;
       return;
     }
@@ -804,7 +804,7 @@ void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, 
   using Kern = void (*)(NlApply<R>, long long, int, int);
   const Kern kern = S <= 32 ? (V ? Kern(nl_apply_kernel<R, 1, true>) : Kern(nl_apply_kernel<R, 1, false>))
                             : (V ? Kern(nl_apply_kernel<R, U, true>) : Kern(nl_apply_kernel<R, U, false>));
-  pdl_launch(kern, dim3(unsigned(blocks)), 128, 0, ctx.stream, a, nitems, nchunks, sl);
+  pdl_launch(true, kern, dim3(unsigned(blocks)), 128, 0, ctx.stream, a, nitems, nchunks, sl);
   ctx.launches++;
 }
 
