@@ -61,7 +61,7 @@ int inqb_ctx_launch_count(inqb_ctx *ctx, long long *count);
  * they carry no rounding bias, and single-precision projector sums; 1 double everywhere; 2
  * double except the last inverse pass of H; 3 as 2 and single for the first forward pass of
  * every transform too (1-3 sum the projections in double); "fft_stages" = 0 (ring depth of the TMA
- * kernels from their shared-memory budget, the default) or 2..8 stages; "overlap_tc" = 1
+ * kernels by pass, line length, precision and set size, the default) or 2..8 stages; "overlap_tc" = 1
  * (default: overlaps of single-precision sets -- inqb_overlap, and the ones inside
  * inqb_orthogonalize and inqb_subspace_diagonalization -- on the tensor cores as split-BF16
  * products with FP32 accumulation and an FP64 sum of the per-SM partials; 16 significant bits
@@ -71,9 +71,10 @@ int inqb_ctx_launch_count(inqb_ctx *ctx, long long *count);
  * for the kernels of other contexts, e.g. small requests next to a large one in a serving loop);
  * "stream_priority" = 0 (default, the device's lowest stream priority) or 1 (its highest: the
  * block scheduler starts this context's pending blocks first); "nl_bulk" = 0 (default: the
- * nonlocal apply, and the projection when it has at least two CTAs per SM, move whole rows of
- * states through shared memory with bulk asynchronous copies), 1 (those forms wherever a row is a
- * multiple of 16 bytes) or -1 (never: register-held gathers); "fft_wide" = 1 (default: the plain streaming
+ * nonlocal apply of rows of at least 256 bytes, and the projection of more than 32 states when it has at least
+ * two CTAs per SM, move whole rows of states through shared memory with bulk asynchronous copies), 1 (those
+ * forms wherever they can; the projection needs rows of 16-byte multiples) or -1 (never: register-held
+ * gathers); "fft_wide" = 1 (default: the plain streaming
  * FFT passes of single-precision sets of at least 64 states move 512-byte rows, 64 states, in three
  * stages at one CTA per SM, unless 64-state tiles would leave more than 8 more empty states in a line's
  * last tile than 32-state tiles) or 0 (256-byte rows, 32 states, as the other passes);
@@ -85,9 +86,9 @@ int inqb_ctx_launch_count(inqb_ctx *ctx, long long *count);
  * one grid line times a block of states);
  * "fp64_mma" = 1 (default: the FP64 products of overlaps of double-precision sets and of every rotation
  * run on the FP64 tensor cores, mma.sync m8n8k4) or 0 (FP64 SIMT fused multiply-adds);
- * "nl_apply_points" = 0 (default: 8) or 1..32 hit points per batch of the bulk-copy nonlocal apply;
+ * "nl_apply_points" = 0 (default: 8, or 16 for many rows of at most 1 KB) or 1..32 hit points per batch of the bulk-copy nonlocal apply;
  * "nl_project_points" = 0 (default: about 16 KB of rows) or 1..32 sphere points per stage of the
- * bulk-copy projection; "nl_project_ranges" = 0 (default: 16) or 1..64 ranges of each sphere's points,
+ * bulk-copy projection; "nl_project_ranges" = 0 (default: 16, or 32 when few projectors would leave SMs idle) or 1..64 ranges of each sphere's points,
  * one CTA each, in the projection (the projection's summation order follows it).  Changing the priority replaces
  * the context's stream (after the work queued on it), so callers query inqb_ctx_stream again. */
 int inqb_ctx_set_option(inqb_ctx *ctx, const char *key, long long value);

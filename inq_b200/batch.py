@@ -32,11 +32,11 @@ DEFAULT_OPTIONS = {"fft_impl": 0, "fft_wide": 1, "fft_flat": 1, "fft_stages": 0,
 #   fft_impl           specialised persistent TMA kernels (0) or the generic kernel (1)
 #   fft_wide           512-byte (64-state) rows in the single-precision streaming passes (1) or 256-byte (0)
 #   fft_flat           y and x passes over flattened (point, state) columns (1) or line x state-block tiles (0)
-#   fft_stages         ring depth of the TMA passes (0: from their shared-memory budget)
+#   fft_stages         ring depth of the TMA passes (0: by pass, line, precision and set size)
 #   nl_bulk            bulk-copy nonlocal kernels by size (0), wherever rows allow (1), never (-1)
-#   nl_apply_points    hit points per batch of the bulk-copy nonlocal apply (0: 8)
+#   nl_apply_points    hit points per batch of the bulk-copy nonlocal apply (0: 8 or 16)
 #   nl_project_points  sphere points per stage of the bulk-copy projection (0: about 16 KB of rows)
-#   nl_project_ranges  ranges of each sphere's points, one CTA each, in the projection (0: 16)
+#   nl_project_ranges  ranges of each sphere's points, one CTA each, in the projection (0: 16 or 32)
 SEARCH_SPACE = (("fft_impl", (0, 1)), ("fft_wide", (1, 0)), ("fft_flat", (1, 0)), ("fft_stages", (0, 2, 3, 4)),
                 ("nl_bulk", (0, 1, -1)),
                 ("nl_apply_points", (0, 4, 16)), ("nl_project_points", (0, 4, 8, 16)),

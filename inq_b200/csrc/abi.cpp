@@ -1985,9 +1985,9 @@ int inqb_subspace_diagonalization(const inqb_hamiltonian *hc, inqb_orbitals *phi
       overlap_dev(*phi, hp.o, d);
     }
     // eigenvalues in ascending order; phi_k <- sum_j V[j][k] phi_j (operations::rotate, rotate.hpp:27-62)
-    if (S <= 13) {
+    if (S <= 13 || S > 4096) {
       // few states: the host's rotations take less time than the device's chain of waves (12 states 0.4 against
-      // 0.5 ms, 16 states 1.1 against 0.65)
+      // 0.5 ms, 16 states 1.1 against 0.65); very many: a wave's rotations would not fit its shared memory
       const auto Hs = download<std::complex<double>>(ctx, d, size_t(S) * S);
       std::vector<std::complex<double>> V(size_t(S) * S);
       hermitian_eigen(S, Hs.data(), eigenvalues, V.data());
