@@ -21,7 +21,7 @@ namespace {
 
 // ------------------------------------------------------------------ Cholesky S = U^H U and X = U^-1
 // (matrix/cholesky.hpp:28-89, invert_triangular.hpp:20-60).  Blocked, 32 x 32 tiles, rows of U from the top:
-// launch k factors the diagonal tile k (every CTA for itself: a serial chain of 32 square roots that is
+// launch k factors the diagonal tile k (every CTA for itself: a serial chain of 32 reciprocals that is
 // shorter than a launch) and solves for one tile of U's row k per CTA, the next launch subtracts the row's
 // products from the tiles below.  Then one CTA per tile column back-substitutes its column of X.
 constexpr int CB = 32;            // tile
@@ -46,9 +46,15 @@ __device__ __forceinline__ double2 csubmulc(double2 a, double2 x, double2 y) {  
 // diagonal tile to D (A is read by the others meanwhile).  The elimination keeps its rows unscaled (row q times
 // 1 / d_qq is subtracted), so the serial chain per row is one reciprocal and one barrier; the square roots of
 // the pivots scale all rows at the end (with the scaling inside the chain a tile took 36 us).
-__global__ void __launch_bounds__(CT) chol_row_kernel(double2 *A, double2 *D, int n, int k, int *bad) {
+// *before: an earlier row had a pivot that is not positive; *after: this one or an earlier one has.  Two flags,
+// so that no launch writes what its other CTAs read; every CTA finds the same pivots, and CTA 0 writes.
+__global__ void __launch_bounds__(CT) chol_row_kernel(double2 *A, double2 *D, int n, int k, const int *before, int *after) {
   __shared__ double2 d[CB][CLD], t[CB][CLD];
-  if (*bad) return;
+  const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
+  if (*before) {
+    if (writer) *after = 1;
+    return;
+  }
   tile_load(d, A, n, k, k);
   const int tj = k + 1 + int(blockIdx.x);
   const bool panel = tj * CB < n;
@@ -57,7 +63,7 @@ __global__ void __launch_bounds__(CT) chol_row_kernel(double2 *A, double2 *D, in
   for (int q = 0; q < CB; q++) {
     const double p = d[q][q].x;  // the tile is Hermitian: the pivot's imaginary part is rounding
     if (!(p > 0.0)) {  // every thread read the same pivot
-      if (threadIdx.x == 0) *bad = 1;
+      if (writer) *after = 1;
       return;
     }
     const double inv = 1.0 / p;
@@ -387,18 +393,22 @@ __global__ void permute_columns_kernel(const double2 *__restrict__ V, const int 
 void launch_cholesky_inverse(Ctx &ctx, int n, double2 *S, double2 *X, int *bad_dev) {
   const int nt = (n + CB - 1) / CB;
   double2 *D = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * size_t(nt) * CB * CB));
+  int *flags = static_cast<int *>(dev_alloc(ctx, sizeof(int) * size_t(nt)));  // what the rows before k found
+  INQB_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * size_t(nt), ctx.stream));
   INQB_CUDA(cudaMemsetAsync(bad_dev, 0, sizeof(int), ctx.stream));
   for (int k = 0; k < nt; k++) {
     const int left = nt - 1 - k;
-    chol_row_kernel<<<left > 0 ? left : 1, CT, 0, ctx.stream>>>(S, D + size_t(k) * CB * CB, n, k, bad_dev);
+    int *after = left > 0 ? flags + k + 1 : bad_dev;
+    chol_row_kernel<<<left > 0 ? left : 1, CT, 0, ctx.stream>>>(S, D + size_t(k) * CB * CB, n, k, flags + k, after);
     LAUNCHED(ctx);
     if (left > 0) {
-      chol_update_kernel<<<left * (left + 1) / 2, CT, 0, ctx.stream>>>(S, n, k, bad_dev);
+      chol_update_kernel<<<left * (left + 1) / 2, CT, 0, ctx.stream>>>(S, n, k, after);
       LAUNCHED(ctx);
     }
   }
   tri_inverse_kernel<<<nt, CT, 0, ctx.stream>>>(S, D, X, n, bad_dev);
   LAUNCHED(ctx);
+  dev_free(ctx, flags);
   dev_free(ctx, D);
 }
 

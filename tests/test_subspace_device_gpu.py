@@ -52,6 +52,24 @@ def test_orthogonalize_refuses_dependent_states(nst):
     assert np.array_equal(phi.matrix(), x)
 
 
+# the failing pivot in the first, a middle and the last tile row, at its first and last row, with up to 12 CTAs per
+# launch and as many launches after the failing one; the context's next call is not affected
+@pytest.mark.parametrize("nst,row", [(400, 0), (400, 31), (400, 32), (129, 63), (129, 100), (129, 127), (129, 128)])
+def test_orthogonalize_refuses_at_any_row(nst, row):
+    import inq_b200 as ib
+    basis, _, x, phi = _set(nst)
+    x[:, row] = 0.0
+    phi.upload(x)
+    for _ in range(3):
+        with pytest.raises(ib.InqbError, match="not positive definite"):
+            ib.orthogonalize(phi)
+    assert np.array_equal(phi.matrix(), x)
+    _, _, y, good = _set(65)
+    ib.orthogonalize(good)
+    got = good.matrix()
+    assert np.abs(basis.volume_element() * (got.conj().T @ got) - np.eye(65)).max() < 1e-12
+
+
 # The device's waves are the host routine's rotations in another order of independent ones: eigenvalues agree
 # to rounding, eigenvectors to rounding over the smallest gap, each up to a phase.  The phase of a vector is
 # that of the off-diagonal element r of its last rotation by about pi / 2 (which swaps two columns), known to
