@@ -42,8 +42,17 @@ GMetric gmetric_of(const Basis &b) {
   return m;
 }
 // factor * (-|G|^2 + gc.G + k2) of a Fourier-space point (fourier_space.hpp:77-125)
-__device__ __forceinline__ double lapl_of(const GMetric &m, int pt, double factor, const double *gc, double k2) {
-  const int row = pt / m.n[2], iz = pt - row * m.n[2], ix = row / m.n[1], iy = row - ix * m.n[1];
+// (32-bit divisions where the point's index allows: 64-bit ones took most of the separate preconditioner's time)
+__device__ __forceinline__ double lapl_of(const GMetric &m, long long pt, double factor, const double *gc, double k2) {
+  int row, iz;
+  if (pt < (1LL << 31)) {
+    row = int(pt) / m.n[2];
+    iz = int(pt) - row * m.n[2];
+  } else {
+    row = int(pt / m.n[2]);
+    iz = int(pt - (long long)row * m.n[2]);
+  }
+  const int ix = row / m.n[1], iy = row - ix * m.n[1];
   auto sym = [](int i, int n) { return i >= (n + 1) / 2 ? i - n : i; };
   const double tp = 6.283185307179586476925286766559;
   const double G0 = tp * sym(ix, m.n[0]), G1 = tp * sym(iy, m.n[1]), G2 = tp * sym(iz, m.n[2]);
@@ -104,7 +113,7 @@ template <typename R> struct SumKinetic {
   double factor, gc[3], k2;
   __device__ void state(int) {}
   __device__ void term(long long p, int s, int S, double (&v)[V]) const {
-    v[0] += lapl_of(m, int(p), factor, gc, k2) * norm2(wide(a[p * S + s]));
+    v[0] += lapl_of(m, p, factor, gc, k2) * norm2(wide(a[p * S + s]));
   }
 };
 
@@ -137,7 +146,7 @@ template <typename R> struct SumResidualKinetic {
   __device__ void term(long long p, int s, int S, double (&v)[V]) const {
     const double zero[3] = {0.0, 0.0, 0.0};
     const double n = norm2(wide(residual<R>(hphi[p * S + s], phi[p * S + s], e)));
-    v[0] += lapl_of(m, int(p), -0.5, zero, 0.0) * n;
+    v[0] += lapl_of(m, p, -0.5, zero, 0.0) * n;
     v[1] += n;
   }
 };
@@ -349,11 +358,10 @@ __global__ void precondition_kernel(GMetric m, const C2<R> *__restrict__ phi, co
   const double zero[3] = {0.0, 0.0, 0.0};
   const long long n = npoints * S;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    // 32-bit point and state indices: 64-bit divisions took most of the separate preconditioner's time
     const long long p = n < (1LL << 31) ? (long long)(uint32_t(i) / uint32_t(S)) : i / S;
     const int s = int(i - p * S);
     const double2 x = wide(residual<R>(hphi[i], phi[i], coef[s]));
-    const double t = lapl_of(m, int(p), -0.5, zero, 0.0) / kin[s];
+    const double t = lapl_of(m, p, -0.5, zero, 0.0) / kin[s];
     const double num = ((8.0 * t + 12.0) * t + 18.0) * t + 27.0;
     const double den = (((16.0 * t + 8.0) * t + 12.0) * t + 18.0) * t + 27.0;
     const double k = num / den;

@@ -120,3 +120,26 @@ def test_state_sums(nst, precision):
     occ = rng.uniform(0.0, 2.0, nst)
     dens = ib.density([phi, b_set], [occ, occ])
     assert np.allclose(dens, (np.abs(a) ** 2) @ occ + (np.abs(b) ** 2) @ occ, rtol=1e-13)
+
+
+# a grid of more than 2^31 points: the coordinates of the last ones need 64-bit indices.  One plane wave e^{iG.r} with
+# G = -(1, 2, 3) 2 pi / L; its kinetic energy is one term, so only the rounding of that term is left
+def test_kinetic_energy_beyond_32_bit_points():
+    import torch
+
+    import inq_b200 as ib
+    n = (1296, 1296, 1280)
+    assert n[0] * n[1] * n[2] > 2 ** 31
+    length = [0.3 * k for k in n]
+    basis = ib.RealSpace(ib.Cell.orthorhombic(*length), sizes=n)
+    data = torch.zeros(n + (1,), dtype=torch.complex64, device="cuda")
+    data[n[0] - 1, n[1] - 2, n[2] - 3, 0] = 2.0
+    torch.cuda.synchronize()
+    phi = ib.OrbitalSet.from_tensor(basis, data, space=ib.FOURIER_SPACE)
+    ham = ib.KSHamiltonian(basis)
+    got = ham.kinetic_expectation_value(phi)
+    g2 = sum((m * 2.0 * np.pi / l) ** 2 for m, l in zip((1, 2, 3), length))
+    want = 0.5 * g2 * 4.0 * np.prod(length) / float(basis.size()) ** 2
+    del ham, phi, data
+    torch.cuda.empty_cache()
+    assert abs(got[0] - want) < 1e-12 * want
