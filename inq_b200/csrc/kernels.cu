@@ -408,17 +408,17 @@ void launch_nl_project(Ctx &ctx, const Basis &b, const Hamiltonian &h, const C2<
   const bool dbl = sizeof(R) == 8 || ctx.mixed_compute != 0;  // double-precision coefficients and sums
   // ranges per sphere (option nl_project_ranges; the summation order follows it)
   int NR = ctx.nl_project_ranges > 0 ? ctx.nl_project_ranges : NLP_RANGES;
-  // bulk form: rows of 16-byte multiples, and (automatic choice) more than 32 states and, with at most 32
-  // ranges, two CTAs per SM; the choice (and so the summation order) follows the device's SM count, not the
-  // grid_sms option.  Fewer states leave most of the bulk form's threads idle: 8 states of 24 projectors
+  // bulk form: rows of 16-byte multiples, and (automatic choice) more than 32 states and two CTAs per SM, with
+  // the ranges the option asks for or, where it leaves them open, at most 32; the choice (and so the summation
+  // order) follows the device's SM count, not the grid_sms option.  Fewer states leave most of the bulk form's threads idle: 8 states of 24 projectors
   // 29 us against 9 in the register form; 50 FP64 states of 12 projectors 19 against 28.
   constexpr int JB = 2;
   const size_t row_bytes = size_t(S) * sizeof(C2<R>);
   const int nchunks = (S + NLA_NT * JB - 1) / (NLA_NT * JB);
   const bool bulk_ok = row_bytes % 16 == 0 && reinterpret_cast<uintptr_t>(psi) % 16 == 0;
-  const bool bulk = bulk_ok && (ctx.nl_bulk > 0 ||
-                                (ctx.nl_bulk == 0 && S > 32 &&
-                                 (long long)P.nproj * std::max(NR, NLP_MAX_RANGES) * nchunks >= 2LL * ctx.device_sms));
+  const int most = ctx.nl_project_ranges > 0 ? NR : std::max(NR, NLP_MAX_RANGES);
+  const bool bulk = bulk_ok && (ctx.nl_bulk > 0 || (ctx.nl_bulk == 0 && S > 32 &&
+                                                    (long long)P.nproj * most * nchunks >= 2LL * ctx.device_sms));
   // register form: two states per lane, or one in lane groups of a power of two
   int sl = 5, K = 2;
   if (S <= 32) {
