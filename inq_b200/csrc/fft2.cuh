@@ -1527,7 +1527,14 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
     ns = 56 * 1024 > fixed + fixed_aux ? int((56 * 1024 - fixed - fixed_aux) / per_stage) : 0;
     ns = ns < 2 || in_l2 ? 2 : (ns > 6 ? 6 : ns);
   }
-  if (ctx.fft_stages > 0) ns = ctx.fft_stages < 2 ? 2 : ctx.fft_stages;
+  if (ctx.fft_stages > 0) {
+    ns = ctx.fft_stages < 2 ? 2 : ctx.fft_stages;
+    // the lengths of has_wide_arith with at least a 256-byte row of states refuse a ring that does not fit (below);
+    // other sets, which ran the generic kernel whatever the depth before they had a pass of their own, take the
+    // deepest ring that fits
+    if (!has_wide_arith(N) || a.S < 256 / int(sizeof(T)))
+      while (ns > 2 && bytes(ns) > ctx.max_smem_optin) ns--;
+  }
   if (gg.cpa) ns = 2;
   gg.stages = ns;
   if (gg.flat) {

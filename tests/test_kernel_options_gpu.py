@@ -37,3 +37,35 @@ def test_projection_form_follows_the_ranges_asked_for(natoms, ranges, bulk):
         ctx.set_option("nl_project_ranges", 0)
     assert not np.array_equal(out[1], out[-1])
     assert np.array_equal(out[0], out[1 if bulk else -1])
+
+
+# ring depths deeper than shared memory holds: line lengths and state counts that only the generic kernel took before
+# their specialised passes still take every depth, and a depth changes no result
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("sizes,nst", [((16, 80, 20), 64), ((100, 20, 16), 64), ((20, 16, 80), 30), ((24, 20, 96), 9),
+                                       ((128, 16, 16), 3)])
+def test_every_ring_depth_is_taken(sizes, nst, precision):
+    ib, basis, ham, phi = _system(nst, 2, sizes, precision)
+    ctx = basis.ctx
+    run = lambda: (ham(phi).matrix(), ib.to_real(ib.to_fourier(phi)).matrix())  # noqa: E731
+    ref = run()
+    try:
+        for depth in (1, 2, 3, 5, 8):
+            ctx.set_option("fft_stages", depth)
+            for got, want in zip(run(), ref):
+                assert np.array_equal(got, want), depth
+    finally:
+        ctx.set_option("fft_stages", 0)
+
+
+# the nine lengths with at least a 256-byte row of states refuse a ring that does not fit, as the option always did
+def test_too_deep_ring_is_refused_for_whole_rows():
+    ib, basis, ham, phi = _system(64, 1, (16, 96, 16), "f32")
+    ctx = basis.ctx
+    ctx.set_option("fft_stages", 8)
+    try:
+        with pytest.raises(ib.InqbError, match="does not fit"):
+            ham(phi)
+    finally:
+        ctx.set_option("fft_stages", 0)
+    ham(phi).matrix()
