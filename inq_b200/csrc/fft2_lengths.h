@@ -50,7 +50,8 @@ struct ZLines {
 };
 inline size_t zlines_smem(int n, int S, int elem_bytes, int lpt, int stages) {
   const size_t tw = size_t(elem_bytes == 8 ? 2 : 1) * n * elem_bytes;
-  return size_t(stages) * lpt * n * S * elem_bytes + tw + ((size_t(lpt) * n * (elem_bytes / 2) + 15) & ~size_t(15)) + 128;
+  const size_t bars = stages < 8 ? 128 : 160;  // two barriers per stage and a flag
+  return size_t(stages) * lpt * n * S * elem_bytes + tw + ((size_t(lpt) * n * (elem_bytes / 2) + 15) & ~size_t(15)) + bars;
 }
 inline ZLines zlines_of(const Ctx &ctx, const Basis &b, int S, int elem_bytes) {
   ZLines z;
@@ -68,6 +69,10 @@ inline ZLines zlines_of(const Ctx &ctx, const Basis &b, int S, int elem_bytes) {
   const size_t top = ctx.max_smem_optin;
   if (zlines_smem(n, S, elem_bytes, int(lpt), 2) > top) return z;
   z.stages = zlines_smem(n, S, elem_bytes, int(lpt), 3) <= top / 2 ? 3 : 2;
+  if (ctx.fft_stages > 0) {  // the depth asked for, as far as it fits (two stages do)
+    z.stages = ctx.fft_stages < 2 ? 2 : ctx.fft_stages;
+    while (z.stages > 2 && zlines_smem(n, S, elem_bytes, int(lpt), z.stages) > top) z.stages--;
+  }
   const size_t smem = zlines_smem(n, S, elem_bytes, int(lpt), z.stages) + 1024;
   const int ctas = int((top + 1024) / smem);
   // 10 to 18 warps per SM whatever the number of CTAs its shared memory holds
