@@ -525,8 +525,9 @@ template <typename R> struct NlApply {
   R vshift;
 };
 // the term's first hit is summed by the caller (fused products); the others follow
-// (VM: with the local potential; a runtime choice cost 177 against 155 us at 96^3 x 256 single)
-template <typename R, bool VM>
+// VM: 0 without the local potential, 1 with it, 2 with it and V + vshift and its product in double (the passes'
+// arithmetic is double then); a runtime choice cost 177 against 155 us at 96^3 x 256 single
+template <typename R, int VM>
 __device__ __forceinline__ C2<R> nl_value(const NlApply<R> &a, long long pt, int s, int h0, int nh, C2<R> o,
                                           const C2<R> (&hc)[4], const C2<R> (&pd)[4]) {
   using T = C2<R>;
@@ -541,7 +542,11 @@ __device__ __forceinline__ C2<R> nl_value(const NlApply<R> &a, long long pt, int
     for (int l = 0; l < 4; l++)
       accv = cadd(accv, cmul(a.hcoef[(long long)h * 4 + l], a.projD[((long long)p * 4 + l) * a.S + s]));
   }
-  if constexpr (VM) o = cscale(o, a.V[pt * a.nspin + a.spin] + a.vshift);
+  if constexpr (VM == 1) o = cscale(o, a.V[pt * a.nspin + a.spin] + a.vshift);
+  if constexpr (VM == 2) {
+    const double v = double(a.V[pt * a.nspin + a.spin]) + double(a.vshift);
+    o = mk<T>(R(double(o.x) * v), R(double(o.y) * v));
+  }
   return cadd(o, a.scaled ? cmul(a.scale, accv) : accv);
 }
 
@@ -550,7 +555,7 @@ __device__ __forceinline__ C2<R> nl_value(const NlApply<R> &a, long long pt, int
 // the coefficient, projection and output reads are all issued together (a two-level dependency instead of
 // point -> CSR -> hit -> projection); splitting the states into chunks keeps the registers low and many
 // warps resident.
-template <typename R, int U, bool VM>
+template <typename R, int U, int VM>
 __global__ void __launch_bounds__(128) nl_apply_kernel(NlApply<R> a, long long nitems, int nchunks, int sl) {
   using T = C2<R>;
   const int S = a.S, SL = 1 << sl;
@@ -600,7 +605,7 @@ __global__ void __launch_bounds__(128) nl_apply_kernel(NlApply<R> a, long long n
 constexpr int NLA_NS = 2;     // stages
 constexpr int NLA_KMAX = 32;  // largest batch (one producer lane per row)
 
-template <typename R, int J, bool BS, bool VM>
+template <typename R, int J, bool BS, int VM>
 __global__ void __launch_bounds__(NLA_NT + 32, sizeof(R) == 4 ? 6 : 3) nl_apply_bulk_kernel(NlApply<R> a, long long nrec,
                                                                                          int KB, int ts, int *err) {
   using T = C2<R>;
@@ -744,6 +749,9 @@ void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, 
   a.nspin = nspin;
   a.spin = spin;
   a.vshift = vshift;
+  // with the local potential: 1, or 2 when the forward pass that multiplies the other points computes in double
+  const int vm = V == nullptr ? 0 : (sizeof(R) == 4 && (ctx.mixed_compute == 1 || ctx.mixed_compute == 2) ? 2 : 1);
+  constexpr int VW = sizeof(R) == 4 ? 2 : 1;  // double sets have no second form
   // bulk form: up to 4 states per compute thread; rows of 16-byte multiples, or sets whose last row's copy
   // ends inside them
   const size_t row_bytes = size_t(S) * sizeof(C2<R>), slot = (row_bytes + 15) & ~size_t(15);
@@ -759,23 +767,24 @@ void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, 
     const size_t smem = size_t(NLA_NS) * KB * (slot + 4 * sizeof(C2<R>) + sizeof(int4)) + 2 * NLA_NS * sizeof(uint64_t) + 16;
     if (smem <= size_t(ctx.max_smem_optin)) {
       const bool bs = row_bytes % 16 == 0 && row_bytes >= 1024;
-      const bool vm = V != nullptr;
       using Kern = void (*)(NlApply<R>, long long, int, int, int *);
-      static const Kern kerns[12] = {
-          nl_apply_bulk_kernel<R, 1, false, false>, nl_apply_bulk_kernel<R, 2, false, false>, nl_apply_bulk_kernel<R, 4, false, false>,
-          nl_apply_bulk_kernel<R, 1, true, false>,  nl_apply_bulk_kernel<R, 2, true, false>,  nl_apply_bulk_kernel<R, 4, true, false>,
-          nl_apply_bulk_kernel<R, 1, false, true>,  nl_apply_bulk_kernel<R, 2, false, true>,  nl_apply_bulk_kernel<R, 4, false, true>,
-          nl_apply_bulk_kernel<R, 1, true, true>,   nl_apply_bulk_kernel<R, 2, true, true>,   nl_apply_bulk_kernel<R, 4, true, true>};
-      // states per thread 1, 2 or 4; rows copied out or stored; with or without the local potential
-      const int ki = (S <= NLA_NT ? 0 : (S <= 2 * NLA_NT ? 1 : 2)) + (bs ? 3 : 0) + (vm ? 6 : 0);
+      static const Kern kerns[18] = {
+          nl_apply_bulk_kernel<R, 1, false, 0>,  nl_apply_bulk_kernel<R, 2, false, 0>,  nl_apply_bulk_kernel<R, 4, false, 0>,
+          nl_apply_bulk_kernel<R, 1, true, 0>,   nl_apply_bulk_kernel<R, 2, true, 0>,   nl_apply_bulk_kernel<R, 4, true, 0>,
+          nl_apply_bulk_kernel<R, 1, false, 1>,  nl_apply_bulk_kernel<R, 2, false, 1>,  nl_apply_bulk_kernel<R, 4, false, 1>,
+          nl_apply_bulk_kernel<R, 1, true, 1>,   nl_apply_bulk_kernel<R, 2, true, 1>,   nl_apply_bulk_kernel<R, 4, true, 1>,
+          nl_apply_bulk_kernel<R, 1, false, VW>, nl_apply_bulk_kernel<R, 2, false, VW>, nl_apply_bulk_kernel<R, 4, false, VW>,
+          nl_apply_bulk_kernel<R, 1, true, VW>,  nl_apply_bulk_kernel<R, 2, true, VW>,  nl_apply_bulk_kernel<R, 4, true, VW>};
+      // states per thread 1, 2 or 4; rows copied out or stored; the local potential
+      const int ki = (S <= NLA_NT ? 0 : (S <= 2 * NLA_NT ? 1 : 2)) + (bs ? 3 : 0) + 6 * vm;
       const Kern kern = kerns[ki];
       int ts = 7;  // threads per row: a power of two from 8 to 128
       while (ts > 3 && (1 << (ts - 1)) >= S) ts--;
       ensure_smem_attr(reinterpret_cast<const void *>(kern), smem);
       // CTAs per SM for this kernel and shared-memory size, computed once under a lock
       static std::mutex mtx;
-      static size_t occ_smem[12] = {};
-      static int occ_per_sm[12] = {};
+      static size_t occ_smem[18] = {};
+      static int occ_per_sm[18] = {};
       int per_sm;
       {
         std::lock_guard<std::mutex> lock(mtx);
@@ -802,8 +811,9 @@ void launch_nl_apply(Ctx &ctx, const Hamiltonian &h, const C2<R> *projD, int S, 
   long long blocks = ((nitems << sl) + 127) / 128;
   if (blocks > 148LL * 48) blocks = 148LL * 48;
   using Kern = void (*)(NlApply<R>, long long, int, int);
-  const Kern kern = S <= 32 ? (V ? Kern(nl_apply_kernel<R, 1, true>) : Kern(nl_apply_kernel<R, 1, false>))
-                            : (V ? Kern(nl_apply_kernel<R, U, true>) : Kern(nl_apply_kernel<R, U, false>));
+  static const Kern few[3] = {nl_apply_kernel<R, 1, 0>, nl_apply_kernel<R, 1, 1>, nl_apply_kernel<R, 1, VW>};
+  static const Kern many[3] = {nl_apply_kernel<R, U, 0>, nl_apply_kernel<R, U, 1>, nl_apply_kernel<R, U, VW>};
+  const Kern kern = S <= 32 ? few[vm] : many[vm];
   pdl_launch(true, kern, dim3(unsigned(blocks)), 128, 0, ctx.stream, a, nitems, nchunks, sl);
   ctx.launches++;
 }

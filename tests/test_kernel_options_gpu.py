@@ -69,3 +69,32 @@ def test_too_deep_ring_is_refused_for_whole_rows():
     finally:
         ctx.set_option("fft_stages", 0)
     ham(phi).matrix()
+
+
+# V + |k|^2 / 2 of the Fourier form at the sphere points, where the nonlocal apply forms it, in the passes' double
+# arithmetic (whole 16-byte rows of at least 256 bytes): V = 1 and a shift of 5e-8 that single precision would drop
+# (an ulp of 1 is 1.2e-7).  The rounding of the stored sets is random, 1e-7 in each of 24^3 * 34 values, 1e-10 in
+# their mean; with the sphere on about half the points (radius 36 in a 72 bohr cell) a dropped shift leaves 2.5e-8.
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("nst", [34, 64])
+def test_fourier_form_keeps_double_arithmetic_at_sphere_points(nst, mode):
+    import inq_b200 as ib
+    rng = np.random.default_rng(nst)
+    n, length = 24, 72.0
+    basis = ib.RealSpace(ib.Cell.cubic(length), sizes=(n, n, n))
+    ham = ib.KSHamiltonian(basis)
+    ham.set_scalar_potential(np.ones((n, n, n)))
+    ham.update_projectors_gaussian(np.array([[36.0, 36.0, 36.0]]), 36.0, 2.0, np.zeros((1, 4, 4)))
+    k = np.sqrt(2.0 * 5e-8)
+    x = rng.standard_normal((n, n, n, nst)) + 1j * rng.standard_normal((n, n, n, nst))
+    f = ib.OrbitalSet.from_array(basis, x, kpoint=(k * length, 0.0, 0.0), space=ib.FOURIER_SPACE, precision=ib.F32)
+    basis.ctx.set_option("mixed_compute", mode)
+    try:
+        got = ham(f).hypercubic().astype(complex)
+    finally:
+        basis.ctx.set_option("mixed_compute", 0)
+    x = f.hypercubic().astype(complex)
+    g = 2.0 * np.pi / length * np.fft.fftfreq(n, 1.0 / n)
+    kin = 0.5 * (g[:, None, None] ** 2 + g[None, :, None] ** 2 + g[None, None, :] ** 2) + g[:, None, None] * k
+    want = (kin + 1.0 + float(np.float32(0.5 * k * k)))[..., None] * x
+    assert abs((x.conj() * (got - want)).sum().real) < 5e-9 * (np.abs(x) ** 2).sum()
