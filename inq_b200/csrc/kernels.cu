@@ -1389,14 +1389,14 @@ __global__ void __launch_bounds__(256, 2) rotate_tiled_kernel(const C2<R> *__res
 // UPPER: Rm is upper triangular, in == out and Sin == Sout.  A CTA takes all output tiles of its 64 points,
 // from the last to the first: tile j needs the input states up to its own last one only, so it skips the
 // zeros below (5/8 of the products at 256 states), and overwrites states that no later tile reads, so no
-// scratch block and copy back are needed.  *skip != 0 leaves the set as it is.
+// scratch block and copy back are needed.  *skip != 0 (when given) leaves the set as it is.
 template <typename R, bool UPPER>
 __global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *in, int Sin, C2<R> *out,
                                                          int Sout, long long npoints, const double2 *__restrict__ Rm,
                                                          double2 alpha, double2 beta, int scaled, int use_beta,
                                                          const int *skip) {
   using T = C2<R>;
-  if (UPPER && *skip) return;
+  if (UPPER && skip && *skip) return;
   constexpr int TP = 64, TJ = 64, KT = 16, LDA = 20, LDB = TJ + 2;
   constexpr int EPC = 16 / int(sizeof(T));  // elements of in per 16-byte copy
   extern __shared__ __align__(16) unsigned char rsm[];
@@ -1551,7 +1551,7 @@ void launch_rotate_to(Ctx &ctx, const C2<R> *in, int Sin, C2<R> *out, int Sout, 
   LAUNCHED(ctx);
 }
 
-// phi <- phi X in place with X upper triangular, unless *skip_dev
+// phi <- phi X in place with X upper triangular, unless skip_dev is given and *skip_dev is set
 template <typename R>
 void launch_rotate_upper(Ctx &ctx, C2<R> *phi, int S, long long npoints, const double2 *X, const int *skip_dev) {
   const size_t smem = 2 * 64 * 20 * sizeof(C2<R>) + 2 * 16 * 66 * sizeof(double2);

@@ -143,3 +143,20 @@ def test_kinetic_energy_beyond_32_bit_points():
     del ham, phi, data
     torch.cuda.empty_cache()
     assert abs(got[0] - want) < 1e-12 * want
+
+
+# few states: the host forms the factor, and the device runs the overlap's two kernels and one rotation (the chain of
+# tiles would add at least three more launches and take longer); more states on either side of the change
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("nst", [1, 2, 16, 49, 50, 51, 52])
+def test_orthogonalize_of_few_states(nst, precision):
+    import inq_b200 as ib
+    basis, _, x, phi = _set(nst, precision=ib.F64 if precision == "f64" else ib.F32)
+    x = phi.matrix().astype(complex)
+    dv = basis.volume_element()
+    ref = x @ np.linalg.inv(np.linalg.cholesky(dv * (x.conj().T @ x)).conj().T)
+    before = basis.ctx.launch_count()
+    ib.orthogonalize(phi)
+    launches = basis.ctx.launch_count() - before
+    assert launches <= 3 if nst <= 50 else launches > 3
+    assert np.linalg.norm(phi.matrix() - ref) < (1e-11 if precision == "f64" else 1e-5) * np.linalg.norm(ref)
