@@ -1386,35 +1386,28 @@ __global__ void __launch_bounds__(256, 2) rotate_tiled_kernel(const C2<R> *__res
 // re.re - im.im into the real part, re.im + im.re into the imaginary): 64 points x 64 output states per
 // CTA of 128 threads, each warp a 32 x 32 block of 8 x 8 fragments; operand tiles double-buffered by
 // cp.async, rows padded (20 elements of in, 66 of R) so that the fragment loads hit distinct banks.
-// UPPER: Rm is upper triangular, in == out and Sin == Sout.  A CTA takes all output tiles of its 64 points,
-// from the last to the first: tile j needs the input states up to its own last one only, so it skips the
-// zeros below (5/8 of the products at 256 states), and overwrites states that no later tile reads, so no
-// scratch block and copy back are needed.  *skip != 0 (when given) leaves the set as it is.
+// One output tile of 64 points from p0 and 64 states from j0.  UPPER: Rm is upper triangular and Sin == Sout, so
+// the tile needs the input states up to its own last one only.
 template <typename R, bool UPPER>
-__global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *in, int Sin, C2<R> *out,
-                                                         int Sout, long long npoints, const double2 *__restrict__ Rm,
-                                                         double2 alpha, double2 beta, int scaled, int use_beta,
-                                                         const int *skip) {
+__device__ __forceinline__ void rotate_tile(const C2<R> *in, int Sin, C2<R> *out, int Sout, long long npoints,
+                                            const double2 *__restrict__ Rm, double2 alpha, double2 beta, int scaled,
+                                            int use_beta, long long p0, int j0) {
   using T = C2<R>;
-  if (UPPER && skip && *skip) return;
   constexpr int TP = 64, TJ = 64, KT = 16, LDA = 20, LDB = TJ + 2;
   constexpr int EPC = 16 / int(sizeof(T));  // elements of in per 16-byte copy
   extern __shared__ __align__(16) unsigned char rsm[];
   T *Abuf = reinterpret_cast<T *>(rsm);                                   // [2][TP][LDA]
   double2 *Bbuf = reinterpret_cast<double2 *>(Abuf + 2 * TP * LDA);       // [2][KT][LDB]
-  const int njt = (Sout + TJ - 1) / TJ;
-  const long long p0 = (long long)(UPPER ? blockIdx.x : blockIdx.x / njt) * TP;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
   const int fk = lane & 3, fs = lane >> 2;
-  const bool whole = (size_t(Sin) * sizeof(T)) % 16 == 0;  // rows of 16-byte multiples; else 8-byte copies
-  for (int jt = UPPER ? njt - 1 : int(blockIdx.x % njt), last = UPPER ? 0 : jt; jt >= last; jt--) {
-  const int j0 = jt * TJ;
+  // rows of 16-byte multiples (the full form is only launched for them); else 8-byte copies
+  const bool whole = (size_t(Sin) * sizeof(T)) % 16 == 0;
   const int kend = UPPER && j0 + TJ < Sin ? j0 + TJ : Sin;
   auto issue = [&](int buf, int k0) {
     T *As = Abuf + buf * TP * LDA;
     double2 *Bs = Bbuf + buf * KT * LDB;
-    if (sizeof(T) == 16 || whole) {
+    if (!UPPER || sizeof(T) == 16 || whole) {
       for (int e = threadIdx.x; e < TP * KT / EPC; e += 128) {
         const int r = e / (KT / EPC), kk = (e % (KT / EPC)) * EPC;
         const long long p = p0 + r;
@@ -1497,7 +1490,29 @@ __global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *in, int Si
           *o = mk<T>(R(w.x), R(w.y));
         }
       }
-  }
+}
+
+// A CTA per tile.  The tile is a function of its own for this kernel's sake: inside the loop over tiles that the
+// triangular form needs, the same code took 3 % longer (64^3 x 128 FP64 1633 against 1680 us, 40^3 x 300 1874 against 1932).
+template <typename R>
+__global__ void __launch_bounds__(128) rotate_mma_kernel(const C2<R> *__restrict__ in, int Sin, C2<R> *__restrict__ out,
+                                                         int Sout, long long npoints, const double2 *__restrict__ Rm,
+                                                         double2 alpha, double2 beta, int scaled, int use_beta) {
+  const int njt = (Sout + 63) / 64;
+  rotate_tile<R, false>(in, Sin, out, Sout, npoints, Rm, alpha, beta, scaled, use_beta, (long long)(blockIdx.x / njt) * 64,
+                        int(blockIdx.x % njt) * 64);
+}
+
+// phi <- phi X, X upper triangular, in place: a CTA takes all output tiles of its 64 points, from the last to the
+// first.  A tile skips the zeros below its columns (5/8 of the products are left at 256 states) and overwrites states
+// that no later tile reads, so no scratch block and copy back are needed.  *skip != 0 (when given) leaves the set as it is.
+template <typename R>
+__global__ void __launch_bounds__(128) rotate_upper_kernel(C2<R> *phi, int S, long long npoints,
+                                                           const double2 *__restrict__ X, const int *skip) {
+  if (skip && *skip) return;
+  for (int jt = (S + 63) / 64 - 1; jt >= 0; jt--)
+    rotate_tile<R, true>(phi, S, phi, S, npoints, X, make_double2(1.0, 0.0), make_double2(0.0, 0.0), 0, 0,
+                         (long long)blockIdx.x * 64, jt * 64);
 }
 
 // out <- alpha (in Rm) + beta out, Rm [Sin][Sout]; in == out (Sin == Sout) rotates in place
@@ -1513,14 +1528,14 @@ void launch_rotate_to(Ctx &ctx, const C2<R> *in, int Sin, C2<R> *out, int Sout, 
     // copied back (the kernel's CTAs for one tile of points read all of its states)
     const size_t tsmem = 2 * 64 * 16 * sizeof(C2<R>) + 2 * 16 * 64 * sizeof(double2);
     const size_t msmem = 2 * 64 * 20 * sizeof(C2<R>) + 2 * 16 * 66 * sizeof(double2);
-    if (ctx.fp64_mma) ensure_smem_attr(reinterpret_cast<const void *>(rotate_mma_kernel<R, false>), msmem);
+    if (ctx.fp64_mma) ensure_smem_attr(reinterpret_cast<const void *>(rotate_mma_kernel<R>), msmem);
     else ensure_smem_attr(reinterpret_cast<const void *>(rotate_tiled_kernel<R>), tsmem);
     auto launch = [&](const C2<R> *src, C2<R> *dst, long long n) {
       const long long nblk = (long long)((Sout + 63) / 64) * ((n + 63) / 64);
       INQB_REQUIRE(nblk < (1LL << 31), INQB_ERR_UNSUPPORTED, "set too large for the rotation grid");
       if (ctx.fp64_mma)
-        rotate_mma_kernel<R, false><<<unsigned(nblk), 128, msmem, ctx.stream>>>(src, Sin, dst, Sout, n, Rdev, alpha, beta,
-                                                                                scaled, use_beta, nullptr);
+        rotate_mma_kernel<R><<<unsigned(nblk), 128, msmem, ctx.stream>>>(src, Sin, dst, Sout, n, Rdev, alpha, beta,
+                                                                         scaled, use_beta);
       else
         rotate_tiled_kernel<R><<<unsigned(nblk), 256, tsmem, ctx.stream>>>(src, Sin, dst, Sout, n, Rdev, alpha, beta,
                                                                           scaled, use_beta);
@@ -1555,11 +1570,10 @@ void launch_rotate_to(Ctx &ctx, const C2<R> *in, int Sin, C2<R> *out, int Sout, 
 template <typename R>
 void launch_rotate_upper(Ctx &ctx, C2<R> *phi, int S, long long npoints, const double2 *X, const int *skip_dev) {
   const size_t smem = 2 * 64 * 20 * sizeof(C2<R>) + 2 * 16 * 66 * sizeof(double2);
-  ensure_smem_attr(reinterpret_cast<const void *>(rotate_mma_kernel<R, true>), smem);
+  ensure_smem_attr(reinterpret_cast<const void *>(rotate_upper_kernel<R>), smem);
   const long long nblk = (npoints + 63) / 64;
   INQB_REQUIRE(nblk < (1LL << 31), INQB_ERR_UNSUPPORTED, "set too large for the rotation grid");
-  rotate_mma_kernel<R, true><<<unsigned(nblk), 128, smem, ctx.stream>>>(
-      phi, S, phi, S, npoints, X, make_double2(1.0, 0.0), make_double2(0.0, 0.0), 0, 0, skip_dev);
+  rotate_upper_kernel<R><<<unsigned(nblk), 128, smem, ctx.stream>>>(phi, S, npoints, X, skip_dev);
   LAUNCHED(ctx);
 }
 
