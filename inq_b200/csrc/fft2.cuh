@@ -1008,11 +1008,14 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
     const CR *lv = linev;
     if constexpr (VAR == MID_KIN || VAR == FWD_LAPLADD) {
       if (gg.flat) {
-        // 32-bit divisions: a view row has fewer than 2^31 words (the host checks it)
-        const int col0 = int(t % gg.nsb) * W, l0 = col0 / a.S;
-        const int last = col0 + W - 1 < int(gg.ncols) ? col0 + W - 1 : int(gg.ncols) - 1;
-        const int nl = last / a.S - l0 + 1, mine = col0 + int(threadIdx.x % W);
-        lv = linev + N * ((mine < last ? mine : last) / a.S - l0);
+        // 32-bit divisions: a view row has fewer than 2^31 words (the host checks it).  With S >= W a tile's columns
+        // lie on at most two lines, and comparisons do for the two divisions (issue-bound: 72^3 x 99 single 137 -> 135.5 us, 96^3 x 110 305 -> 302)
+        const int col0 = int(t % gg.nsb) * W, l0 = col0 / a.S, o0 = col0 - l0 * a.S;  // o0: columns of l0 before the tile's
+        const int left = int(gg.ncols) - 1 - col0, last = left < W - 1 ? left : W - 1;  // last column of the tile
+        const int w = int(threadIdx.x % W), mine = w < last ? w : last;
+        const bool few = a.S < W;
+        const int nl = few ? (o0 + last) / a.S + 1 : (o0 + last >= a.S ? 2 : 1);
+        lv = linev + N * (few ? (o0 + mine) / a.S : (o0 + mine >= a.S ? 1 : 0));
         for (int e = threadIdx.x; e < nl * N; e += NT) {
           const int l = l0 + e / N;  // x-line (y, z) = (l / nz, l % nz)
           const int ly = l / g.n[2];

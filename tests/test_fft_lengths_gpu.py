@@ -55,3 +55,27 @@ def test_transforms_against_numpy(sizes, nst, precision, tol):
     assert _rel(f.hypercubic(), np.fft.fftn(phi.hypercubic().astype(complex), axes=(0, 1, 2))) < tol
     assert _rel(ib.to_real(f).hypercubic(), phi.hypercubic()) < 2 * tol
     assert _rel(ib.to_real(f, normalize=False).hypercubic() / basis.size(), phi.hypercubic()) < 2 * tol
+
+
+# x passes over flattened columns with state counts around the tile widths (16 double, 32 single): a column's factors
+# are those of its own line, whether a tile's columns lie on one line, on two or on many; the bounds are those above
+@pytest.mark.parametrize("precision,tol", [("f64", 2e-14), ("f32", 2e-5)])
+@pytest.mark.parametrize("nst", [2, 15, 16, 17, 31, 32, 33, 47, 62])
+def test_kinetic_factors_around_tile_widths(nst, precision, tol):
+    import inq_b200 as ib
+    rng = np.random.default_rng(nst)
+    n = (24, 9, 10)
+    prec = ib.F64 if precision == "f64" else ib.F32
+    basis = ib.RealSpace(ib.Cell.orthorhombic(*[0.3 * x for x in n]), sizes=n)
+    ham = ib.KSHamiltonian(basis)
+    ham.set_scalar_potential(rng.standard_normal(n))
+    x = rng.standard_normal((basis.size(), nst)) + 1j * rng.standard_normal((basis.size(), nst))
+    for space in (ib.REAL_SPACE, ib.FOURIER_SPACE):
+        phi = ib.OrbitalSet.from_array(basis, x, kpoint=(0.1, 0.0, 0.2), space=space, precision=prec)
+        got = ham(phi).matrix()
+        ham.set_option("fft_impl", 1)
+        ref = ham(phi).matrix()
+        ham.set_option("fft_impl", -1)
+        assert _rel(got, ref) < tol
+        # every state by itself: bounds on the whole set could hide one column's factors
+        assert (np.linalg.norm(got - ref, axis=0) < 2 * tol * np.linalg.norm(ref, axis=0)).all()
