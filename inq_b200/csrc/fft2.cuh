@@ -1513,7 +1513,7 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
   //  * other single-precision passes and wider arithmetic: about 56 KB per CTA (four per SM), two stages for sets
   //    that stay in L2 (as fast alone, and the CTAs find room beside the previous pass's last ones).
   constexpr int NTC = threads_of<R, CR, N, VAR, WIDE>();
-  const bool in_l2 = size_t(b.npoints) * a.S * sizeof(T) <= (size_t(128) << 20);
+  const bool in_l2 = stays_in_l2(b, a.S, int(sizeof(T)));
   auto bytes = [&](int n) { return per_stage * n + fixed_aux + fixed; };
   int ns;
   if (WIDE) {
@@ -1677,7 +1677,8 @@ template <typename R, int N>
 void launch_n(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg, int var) {
   if (gg.axis == 2 && (sizeof(R) == 8 || single_arith(ctx, a, var))) {
     const ZLines z = zlines_of(ctx, b, a.S, int(sizeof(C2<R>)));
-    if (z.lpt > 0) {
+    const bool tiles = sizeof(R) == 4 && base_var(var) == INV_FINAL && final_tiles(b, N, a.S);
+    if (z.lpt > 0 && !tiles) {
       switch (var) {
         case FWD_STORE: launch_zlines<R, N, FWD_STORE>(ctx, b, a, z); return;
         case INV_STORE: launch_zlines<R, N, INV_STORE>(ctx, b, a, z); return;

@@ -19,6 +19,11 @@ namespace v2 {
   X(72, 8, 9) X(75, 5, 15) X(80, 8, 10) X(81, 9, 9) X(84, 7, 12) X(90, 9, 10) X(96, 8, 12) X(98, 7, 14)  \
   X(100, 10, 10) X(105, 7, 15) X(108, 9, 12) X(112, 8, 14) X(120, 8, 15) X(126, 9, 14) X(128, 8, 16)
 
+// A set small enough to stay in L2 from one pass to the next
+inline bool stays_in_l2(const Basis &b, int S, int elem_bytes) {
+  return size_t(b.npoints) * S * elem_bytes <= (size_t(128) << 20);
+}
+
 // N2 of a specialised length, 0 for the others
 inline int split_n2(int n) {
   switch (n) {
@@ -82,6 +87,16 @@ inline ZLines zlines_of(const Ctx &ctx, const Basis &b, int S, int elem_bytes) {
   if (items < z.threads) z.threads = int((items + 31) / 32 * 32);
   z.lpt = int(lpt);
   return z;
+}
+
+// Final passes of single-precision sets beyond L2 that keep the line tiles although their other z passes take whole
+// lines: three transits, whose second input a tile brings in by TMA, and the whole-line kernel reads it with its
+// registers' loads.  H single, whole lines against tiles in the final pass: 96^3 x 44 815 -> 730 us, x 62 1024 -> 957,
+// 72^3 x 62 462 -> 438, x 180 1245 -> 1180, 64^3 x 190 872 -> 833, 48^3 x 180 403 -> 374; the same at 96^3 x 110 and more.
+// Not at 80 or 90 points (80^3 x 40 446 -> 478 us, 90^3 x 34 598 -> 645) nor at 120 (x 34 1318 -> 1433: its second
+// tiles have a single buffer), not in L2 (48^3 x 80 176 -> 197), and not in double (96^3 x 62 1797 -> 1880).
+inline bool final_tiles(const Basis &b, int n, int S) {
+  return has_wide_arith(n) && n <= 96 && S >= 32 && S % 2 == 0 && !stays_in_l2(b, S, 8);
 }
 
 // whether a specialised pass moves this set along `axis`, given that it computes in the storage type

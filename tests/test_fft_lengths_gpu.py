@@ -79,3 +79,27 @@ def test_kinetic_factors_around_tile_widths(nst, precision, tol):
         assert _rel(got, ref) < tol
         # every state by itself: bounds on the whole set could hide one column's factors
         assert (np.linalg.norm(got - ref, axis=0) < 2 * tol * np.linalg.norm(ref, axis=0)).all()
+
+
+# single-precision sets beyond L2 (128 MB) whose final pass keeps line tiles while the other z passes take whole lines:
+# the operator and its Horner step, with either arithmetic of the final pass, against the generic kernel
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("sizes,nst", [((48, 64, 96), 62), ((40, 72, 72), 90), ((64, 96, 48), 58)])
+def test_final_tiles_of_large_single_sets(sizes, nst, mode):
+    import inq_b200 as ib
+    rng = np.random.default_rng(nst)
+    basis = ib.RealSpace(ib.Cell.orthorhombic(*[0.3 * x for x in sizes]), sizes=sizes)
+    assert basis.size() * nst * 8 > 128 << 20
+    ham = ib.KSHamiltonian(basis)
+    ham.set_scalar_potential(rng.standard_normal(sizes))
+    x = rng.standard_normal((basis.size(), nst), dtype=np.float32) + 1j * rng.standard_normal((basis.size(), nst), dtype=np.float32)
+    phi = ib.OrbitalSet.from_array(basis, x, kpoint=(0.1, 0.0, 0.2), precision=ib.F32)
+    basis.ctx.set_option("mixed_compute", mode)
+    try:
+        got = ham(phi).matrix(), ib.exponential(ham, -0.002j, phi).matrix()
+        ham.set_option("fft_impl", 1)
+        ref = ham(phi).matrix(), ib.exponential(ham, -0.002j, phi).matrix()
+    finally:
+        basis.ctx.set_option("mixed_compute", 0)
+    for a, b in zip(got, ref):
+        assert _rel(a, b) < 2e-5
