@@ -417,7 +417,8 @@ void launch_jacobi(Ctx &ctx, int n, double2 *A, double2 *V, double *w_dev) {
   double2 *B = static_cast<double2 *>(dev_alloc(ctx, sizeof(double2) * size_t(n) * n));
   double *norms = static_cast<double *>(dev_alloc(ctx, sizeof(double) * 3 * 16));
   const size_t smem = 2 * sizeof(Rot) * size_t(n / 2 + 1);
-  INQB_REQUIRE(smem <= ctx.max_smem_optin, INQB_ERR_UNSUPPORTED, "too many states for the eigen-decomposition");
+  INQB_REQUIRE(smem + sizeof(double) * EIG_THREADS <= ctx.max_smem_optin, INQB_ERR_UNSUPPORTED,
+               "too many states for the eigen-decomposition");  // beside the kernel's sums in static shared memory
   ensure_smem_attr(reinterpret_cast<const void *>(jacobi_kernel), smem);
   INQB_CUDA(cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};

@@ -160,3 +160,56 @@ def test_orthogonalize_of_few_states(nst, precision):
     launches = basis.ctx.launch_count() - before
     assert launches <= 3 if nst <= 50 else launches > 3
     assert np.linalg.norm(phi.matrix() - ref) < (1e-11 if precision == "f64" else 1e-5) * np.linalg.norm(ref)
+
+
+# more rows of 64 points than CTAs are resident (444 or 592 on a B200) and several tiles of states: the triangular
+# rotation works in place, each CTA on its own points
+@pytest.mark.parametrize("precision,nst,tol", [("f64", 200, 1e-12), ("f32", 200, 2e-5), ("f32", 131, 2e-5)])
+def test_orthogonalize_many_points(nst, precision, tol):
+    import inq_b200 as ib
+    basis, _, x, phi = _set(nst, sizes=(40, 40, 42), precision=ib.F64 if precision == "f64" else ib.F32)
+    dv = basis.volume_element()
+    x = phi.matrix().astype(complex)
+    ref = x @ np.linalg.inv(np.linalg.cholesky(dv * (x.conj().T @ x)).conj().T)
+    ib.orthogonalize(phi)
+    assert np.linalg.norm(phi.matrix() - ref) < tol * np.linalg.norm(ref)
+
+
+# the SIMT products: the full rotation, once the host knows that there is a factor
+@pytest.mark.parametrize("precision,nst,tol", [("f64", 33, 1e-11), ("f64", 100, 1e-11), ("f32", 33, 1e-5), ("f32", 64, 1e-5)])
+def test_orthogonalize_without_fp64_tensor_cores(precision, nst, tol):
+    import inq_b200 as ib
+    basis, _, x, phi = _set(nst, precision=ib.F64 if precision == "f64" else ib.F32)
+    dv = basis.volume_element()
+    x = phi.matrix().astype(complex)
+    ref = x @ np.linalg.inv(np.linalg.cholesky(dv * (x.conj().T @ x)).conj().T)
+    basis.ctx.set_option("fp64_mma", 0)
+    try:
+        ib.orthogonalize(phi)
+        assert np.linalg.norm(phi.matrix() - ref) < tol * np.linalg.norm(ref)
+        x[:, nst // 2] = 0.0
+        phi.upload(x)
+        held = phi.matrix()
+        with pytest.raises(ib.InqbError, match="not positive definite"):
+            ib.orthogonalize(phi)
+        assert np.array_equal(phi.matrix(), held)
+    finally:
+        basis.ctx.set_option("fp64_mma", 1)
+
+
+# more than 1024 states: several rounds of a block's threads over a wave's rotations, whose table is larger than the
+# 48 KB a kernel may have without asking.  Against numpy: eigenvalues, orthonormal states, a diagonal matrix
+def test_subspace_diagonalization_of_many_states():
+    import inq_b200 as ib
+    nst = 1030
+    basis, rng, x, phi = _set(nst, sizes=(12, 10, 12))
+    ham = ib.KSHamiltonian(basis)
+    ham.set_scalar_potential(rng.standard_normal(basis.sizes))
+    ib.orthogonalize(phi)
+    w = np.linalg.eigvalsh(ib.overlap(phi, ham(phi)))
+    eig = ham.subspace_diagonalization(phi)
+    norm = np.abs(w).max()
+    assert np.abs(eig - w).max() < 100 * EPS * norm * nst ** 0.5
+    H = ib.overlap(phi, ham(phi))
+    assert np.linalg.norm(H - np.diag(eig)) < 1e-12 * np.linalg.norm(H)
+    assert np.abs(ib.overlap(phi) - np.eye(nst)).max() < 1e-11
