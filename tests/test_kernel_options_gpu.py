@@ -98,3 +98,25 @@ def test_fourier_form_keeps_double_arithmetic_at_sphere_points(nst, mode):
     kin = 0.5 * (g[:, None, None] ** 2 + g[None, :, None] ** 2 + g[None, None, :] ** 2) + g[:, None, None] * k
     want = (kin + 1.0 + float(np.float32(0.5 * k * k)))[..., None] * x
     assert abs((x.conj() * (got - want)).sum().real) < 5e-9 * (np.abs(x) ** 2).sum()
+
+
+# double-precision arithmetic over single-precision sets with fewer states than a 256-byte row, whose flattened
+# tiles lie on several lines: against the generic kernel (single-precision arithmetic; 2e-6 for both, as the parity
+# tests take)
+@pytest.mark.parametrize("mode", [1, 2, 3])
+@pytest.mark.parametrize("sizes,nst", [((24, 24, 24), 1), ((32, 24, 40), 2), ((48, 24, 32), 9), ((24, 40, 64), 16),
+                                       ((24, 72, 24), 31)])
+def test_wide_arithmetic_of_few_states(sizes, nst, mode):
+    ib, basis, ham, phi = _system(nst, 3, sizes, "f32")
+    ctx = basis.ctx
+    f = ib.to_fourier(phi)
+    ctx.set_option("mixed_compute", mode)
+    try:
+        for s in (phi, f):
+            got = ham(s).matrix()
+            ham.set_option("fft_impl", 1)
+            ref = ham(s).matrix()
+            ham.set_option("fft_impl", -1)
+            assert np.linalg.norm(got - ref) < 2e-6 * np.linalg.norm(ref)
+    finally:
+        ctx.set_option("mixed_compute", 0)
