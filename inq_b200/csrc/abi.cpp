@@ -278,7 +278,7 @@ void check_kernel_option(const Ctx &ctx, const std::string &k, long long value) 
   if (k == "nl_apply_points" || k == "nl_project_points")
     INQB_REQUIRE(value >= 0 && value <= 32, INQB_ERR_ARG, k + " is 0 (automatic) or 1..32");
   if (k == "nl_project_ranges")
-    INQB_REQUIRE(value >= 0 && value <= 64, INQB_ERR_ARG, "nl_project_ranges is 0 (16) or 1..64");
+    INQB_REQUIRE(value >= 0 && value <= 64, INQB_ERR_ARG, "nl_project_ranges is 0 (16 or 32) or 1..64");
 }
 
 // The Hamiltonian's kernel-option overrides (inqb_hamiltonian_set_option) in force on its context for

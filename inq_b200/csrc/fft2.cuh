@@ -1009,8 +1009,9 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
     if constexpr (VAR == MID_KIN || VAR == FWD_LAPLADD) {
       if (gg.flat) {
         // 32-bit divisions: a view row has fewer than 2^31 words (the host checks it).  With S >= W a tile's columns
-        // lie on at most two lines, and comparisons do for the two divisions (issue-bound: 72^3 x 99 single 137 -> 135.5 us, 96^3 x 110 305 -> 302)
-        const int col0 = int(t % gg.nsb) * W, l0 = col0 / a.S, o0 = col0 - l0 * a.S;  // o0: columns of l0 before the tile's
+        // lie on at most two lines, and comparisons do for the two divisions per column (issue-bound: 72^3 x 99 single
+        // 137 -> 135.5 us, 96^3 x 110 305 -> 302).  o0: columns of line l0 before the tile's
+        const int col0 = int(t % gg.nsb) * W, l0 = col0 / a.S, o0 = col0 - l0 * a.S;
         const int left = int(gg.ncols) - 1 - col0, last = left < W - 1 ? left : W - 1;  // last column of the tile
         const int w = int(threadIdx.x % W), mine = w < last ? w : last;
         const bool few = a.S < W;
@@ -1165,11 +1166,15 @@ __global__ void __launch_bounds__(block_threads_of<R, CR, N, VAR, WIDE>(), min_c
 // warp stores consecutive elements); the second inputs of an epilogue are read there the same way, before
 // the step's shared-memory loads, so they need no tile of their own.
 //
-// Bound by HBM: one transit in and one out (and the second inputs).  Two stages per CTA and 10 to 18 warps
-// per SM cover the latency; see zlines_of for the chunk and thread counts.  Measured: 72^3 x 99 single,
-// forward 206 -> 95 us (6.2 TB/s) and final 354 -> 183 us against the 8-byte copies; 40^3 x 33 double, forward
-// 22.8 -> 12.4 and final Horner pass 46.7 -> 31.0 us against 16-state tiles (48 slots for 33 states).  Rows
-// that are whole 256-byte tiles keep the TMA tiles of fft2_kernel, which leave nothing empty either.
+// Bound by HBM: one transit in and one out (and the second inputs).  Measured: 72^3 x 99 single, forward 206 -> 95 us
+// (6.2 TB/s) and final 354 -> 183 us against the 8-byte copies; 40^3 x 33 double, forward 22.8 -> 12.4 and final
+// Horner pass 46.7 -> 31.0 us against 16-state tiles (48 slots for 33 states).  zlines_of has the chunk and thread
+// counts, which follow shared memory alone.  The forward and plain inverse kernels (48 to 108 registers a thread)
+// come close to its 10 to 18 warps per SM; the final ones do not: in double they take 99 to 168 registers, so 40^3 x 33
+// (224 threads) runs one CTA per SM where its shared memory would hold three, 54 x 60 x 45 x 50 (288) one of two, and the
+// CTAs beyond those resident follow when they end; natural-order final passes in double spill besides (300 bytes at 75,
+// 105 and 120 points, 104 to 324 at 84, 96, 98, 108, 112, 126 and 128).  Rows that are whole 256-byte tiles keep the
+// TMA tiles of fft2_kernel, which leave nothing empty either, and so do the final passes of final_tiles.
 struct GeomZ {
   long long lines;           // nx * ny
   int lpt, stages;
@@ -1501,10 +1506,11 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
   const size_t fixed_aux = gg.aux_single ? naux * TILE_BYTES : 0;
   // Ring depth.  What counts is the warps per SM that cover the arithmetic's latency, then the bytes in flight;
   // measured per pass (us, one transit in and out at 6.4 TB/s in brackets):
-  //  * double: two stages, so that four to six CTAs share an SM (fwd/inv y pass 60^3 x 64 95/98 -> 81/74 [69],
-  //    120^3 x 64 630/622 -> 576/564 [549]; final pass, two tiles per stage, 64^3 x 128 345 -> 252, 48^3 x 128
-  //    183 -> 113); three in the streaming passes of lines with one first-step item per thread (64, 96 and 128
-  //    points: 96^3 x 128 554/547 with three, 604/597 with two), and in their kinetic pass of sets beyond L2;
+  //  * double: two stages, so that four to six CTAs share an SM (fwd/inv y pass 120^3 x 64 630/622 -> 576/564 [549];
+  //    final pass, two tiles per stage, 64^3 x 128 345 -> 252, 48^3 x 128 183 -> 113); three where the first step has
+  //    exactly one item per thread (50, 60, 64, 70, 80, 84, 90, 96, 98, 100, 108, 112, 126 and 128 points: 96^3 x 128
+  //    554/547 with three, 604/597 with two), and in the kinetic pass of 64 points of sets beyond L2.  A transform alone
+  //    is 1 to 2 % faster with six at 40 and 48 points beyond L2 (48^3 x 128 253 against 247), H slower (497 against 502);
   //  * single, 512-byte rows: three stages for sets that stay in L2 (two to three CTAs per SM up to 72 points:
   //    48^3 x 97 37/36 with six stages, 26/24 with three [27]), four for larger ones while they fit 150 KB
   //    (72^3 x 250 276/269 with three, 240/248 with four [232]), three up to 204 KB (120^3 x 64 350/336 with
@@ -1587,15 +1593,15 @@ void launch_kernel(Ctx &ctx, const Basis &b, const PassArgs<R> &a, Geom2 gg) {
   const TC *tw = reinterpret_cast<const TC *>(sizeof(CR) == 8 ? b.tw64[gg.axis] : b.tw32[gg.axis]);
   // sets beyond L2 start their passes the ordinary way: CTAs that come early settle unevenly in the room the
   // previous pass leaves, and these passes are long enough for that to cost more than the launch gap (H at
-  // 64^3 x 128 FP64 1202 -> 1072 us, 96^3 x 120 single 1625 -> 1592, 96^3 x 256 single 3492 -> 3456)
+  // 64^3 x 128 FP64 1202 -> 1072 us, 96^3 x 120 single 1625 -> 1592)
   pdl_launch(in_l2, kern, dim3(unsigned(grid)), NT, smem, ctx.stream, mi, mo, mx, mb, a, gg, tw, ctx.d_err);
   ctx.launches++;
 }
 
-// The plain streaming passes of single-precision sets of at least 64 states run with 512-byte rows
-// (64 states) in three stages, one CTA per SM (context option fft_wide, default 1).  Measured at
-// 96^3 x 256: 0.571 ms per pass against 0.633 ms with 256-byte rows at four CTAs per SM (6.35 against
-// 5.72 TB/s).  The same shape made the kinetic pass slower, and double-precision passes (32 states,
+// The plain streaming passes of single-precision sets run with 512-byte rows (64 states or flattened columns; context
+// option fft_wide, default 1; launch_n says when) in two to four stages, one to three CTAs per SM (launch_kernel).
+// Measured at 96^3 x 256, three stages, one CTA: 0.571 ms per pass against 0.633 ms with 256-byte rows at four CTAs per
+// SM (6.35 against 5.72 TB/s).  The same shape made the kinetic pass slower, and double-precision passes (32 states,
 // one CTA of 256 threads per SM) much slower (1.66 against 1.15 ms), so those keep 256-byte rows.
 inline bool wide_var(int var) { return var == FWD_STORE || var == INV_STORE || var == FWD_PERM || var == INV_PERM; }
 
@@ -1669,6 +1675,8 @@ void launch_zlines(Ctx &ctx, const Basis &b, const PassArgs<R> &a, const ZLines 
   long long grid = (long long)(ctas < 1 ? 1 : (ctas > 8 ? 8 : ctas)) * ctx.num_sms;
   if (grid > tiles) grid = tiles;
   const T *tw = reinterpret_cast<const T *>(sizeof(R) == 8 ? b.tw64[2] : b.tw32[2]);
+  // an early start whatever the set's size: beyond L2 it gains or costs less than 1 % of H (72^3 x 31 double 460 against
+  // 466 us without, 96^3 x 62 1797 against 1806, 64^3 x 79 724 against 705; single 72^3 x 180 1205 against 1207)
   pdl_launch(true, kern, dim3(unsigned(grid)), z.threads + 32, smem, ctx.stream, a, gz, tw, ctx.d_err);
   ctx.launches++;
 }

@@ -80,7 +80,7 @@ inline ZLines zlines_of(const Ctx &ctx, const Basis &b, int S, int elem_bytes) {
   }
   const size_t smem = zlines_smem(n, S, elem_bytes, int(lpt), z.stages) + 1024;
   const int ctas = int((top + 1024) / smem);
-  // 10 to 18 warps per SM whatever the number of CTAs its shared memory holds
+  // 10 to 18 warps per SM, by the CTAs that shared memory would hold; registers allow fewer in most final passes in double
   const int most = elem_bytes == 16 ? 320 : 480;
   z.threads = ctas <= 1 ? most : (ctas == 2 ? 256 : (ctas == 3 ? 192 : 128));
   const long long items = lpt * S * (n2 > n / n2 ? n2 : n / n2);

@@ -71,15 +71,15 @@ struct Ctx {
   std::vector<cudaStream_t> aux;        // fork streams of batched calls
   std::vector<cudaEvent_t> aux_events;  // [0] fork point, [1..] joins
   int fft_impl = 0;          // 0: specialised TMA kernels where available, 1: generic kernel only
-  int fft_stages = 0;        // shared-memory ring depth of the TMA FFT kernels (0: from the memory budget)
+  int fft_stages = 0;        // shared-memory ring depth of the TMA FFT kernels (0: by pass, line, precision and set size)
   int mixed_compute = 0;     // butterfly arithmetic of single-precision orbitals (see inqb_ctx_set_option)
   int overlap_tc = 1;        // overlaps of single-precision sets on the tensor cores (split BF16)
   int nl_bulk = 0;           // nonlocal kernels: 0 automatic, 1 bulk-copy forms wherever they apply, -1 never
   int fft_wide = 1;          // single-precision FFT passes without a second input: 512-byte rows (64 states)
   int fft_flat = 1;          // y and x FFT passes over flattened (point, state) columns (option fft_flat)
-  int nl_project_ranges = 0; // ranges of each sphere's points in the projection (0: 16)
+  int nl_project_ranges = 0; // ranges of each sphere's points in the projection (0: 16, 32 for few projectors)
   int fp64_mma = 1;          // FP64 overlaps on the FP64 tensor-core path (mma.sync m8n8k4) or SIMT (0)
-  int nl_apply_points = 0;   // hit points per batch of the bulk-copy nonlocal apply (0: 8)
+  int nl_apply_points = 0;   // hit points per batch of the bulk-copy nonlocal apply (0: 8 or 16)
   int nl_project_points = 0; // sphere points per stage of the bulk-copy projection (0: about 16 KB of rows)
   int stream_priority = 0;   // 0: the device's lowest stream priority, 1: its highest
   void *noalloc_partial = nullptr;  // device address of noalloc.cu's fixed partial-sum array on this device

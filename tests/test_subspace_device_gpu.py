@@ -213,3 +213,17 @@ def test_subspace_diagonalization_of_many_states():
     H = ib.overlap(phi, ham(phi))
     assert np.linalg.norm(H - np.diag(eig)) < 1e-12 * np.linalg.norm(H)
     assert np.abs(ib.overlap(phi) - np.eye(nst)).max() < 1e-11
+
+
+# norms (a set with itself, its own sum) against the same set under another address and numpy: all terms are positive,
+# so 1e-14 is about 50 roundings of sums that add in groups
+@pytest.mark.parametrize("nst", [1, 8, 9, 40, 256, 300, 600])
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+def test_norms_of_a_set(nst, precision):
+    import inq_b200 as ib
+    basis, _, _, phi = _set(nst, sizes=(9, 7, 5), precision=ib.F64 if precision == "f64" else ib.F32)
+    n = ib.overlap_diagonal(phi)
+    want = basis.volume_element() * (np.abs(phi.matrix().astype(complex)) ** 2).sum(0)
+    assert np.all(n.imag == 0.0)
+    assert np.allclose(n.real, want, rtol=1e-14, atol=0.0)
+    assert np.allclose(ib.overlap_diagonal(phi, phi.copy()).real, n.real, rtol=1e-14, atol=0.0)
