@@ -61,7 +61,9 @@ int inqb_ctx_launch_count(inqb_ctx *ctx, long long *count);
  * they carry no rounding bias, and single-precision projector sums; 1 double everywhere; 2
  * double except the last inverse pass of H; 3 as 2 and single for the first forward pass of
  * every transform too (1-3 sum the projections in double); "fft_stages" = 0 (ring depth of the TMA
- * kernels by pass, line length, precision and set size, the default) or 2..8 stages; "overlap_tc" = 1
+ * kernels by pass, line length, precision and set size, the default) or 1..8 stages (1 is 2; a depth that does not
+ * fit shared memory is an error for line lengths 24, 32, 40, 48, 64, 72, 96, 120 and 128 with at least a 256-byte
+ * row of states, and the deepest that fits elsewhere and in whole-line z passes); "overlap_tc" = 1
  * (default: overlaps of single-precision sets -- inqb_overlap, and the ones inside
  * inqb_orthogonalize and inqb_subspace_diagonalization -- on the tensor cores as split-BF16
  * products with FP32 accumulation and an FP64 sum of the per-SM partials; 16 significant bits
@@ -75,14 +77,15 @@ int inqb_ctx_launch_count(inqb_ctx *ctx, long long *count);
  * two CTAs per SM, move whole rows of states through shared memory with bulk asynchronous copies), 1 (those
  * forms wherever they can; the projection needs rows of 16-byte multiples) or -1 (never: register-held
  * gathers); "fft_wide" = 1 (default: the plain streaming
- * FFT passes of single-precision sets of at least 64 states move 512-byte rows, 64 states, in three
- * stages at one CTA per SM, unless 64-state tiles would leave more than 8 more empty states in a line's
- * last tile than 32-state tiles) or 0 (256-byte rows, 32 states, as the other passes);
+ * FFT passes of single-precision sets move 512-byte rows, 64 states or columns: y and x passes over flattened columns,
+ * and line tiles of at least 64 states unless 64-state tiles would leave more than 8 more empty states in a line's
+ * last tile than 32-state tiles) or 0 (256-byte rows, as the other passes);
  * "fft_flat" = 1 (default: the y and x passes tile the flattened [nx][ny][nz*S] and [nx][ny*nz*S] views
  * of a set, so every row holds a full tile width of (point, state) columns whatever the state count,
  * odd and small counts included, when nz*S elements are a multiple of 16 bytes and the state rows are not
  * already whole 512-byte rows; the z passes take whole lines with all their states, one contiguous chunk,
- * when the state rows are not whole 256-byte rows and two chunks fit a CTA's shared memory) or 0 (tiles of
+ * when the state rows are not whole 256-byte rows and two chunks fit a CTA's shared memory, but for some final passes
+ * of single-precision sets beyond L2) or 0 (tiles of
  * one grid line times a block of states);
  * "fp64_mma" = 1 (default: the FP64 products of overlaps of double-precision sets and of every rotation
  * run on the FP64 tensor cores, mma.sync m8n8k4) or 0 (FP64 SIMT fused multiply-adds);

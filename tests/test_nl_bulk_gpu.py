@@ -10,7 +10,7 @@ bytes, -1 never).  Forced on against forced off, on small systems:
   hits) H|psi> also matches the oracle to 1e-12;
 * the Taylor exponential, whose apply also updates two accumulators, agrees to 1e-13;
 * a single-precision set with an odd state count (rows of 8-byte multiples) takes the register
-  forms under either setting and gives bitwise the same result.
+  projection under either setting, and its apply gives bitwise the same result in both forms.
 """
 
 import numpy as np
